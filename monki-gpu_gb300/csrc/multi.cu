@@ -410,10 +410,10 @@ void run(Multi& m, const std::vector<Controls>& ctl) {
                     if (!ctl[size_t(g.members[q])].count || !live) continue;
                     const SceneEntry<T>& E = host[q];
                     cudaStream_t t = m.tail_streams[used++ % m.tail_streams.size()];
-                    const unsigned blocks = unsigned(std::max<uint64_t>(1, (live + 255) / 256));
+                    const unsigned blocks = unsigned(std::max<uint64_t>(1, (live + 63) / 64));
                     check(launch_tail<T>(E.s, E.ctl, E.dv, E.P, E.banks, E.W, guide, 0u, true, m.failure, E.counters,
                                          m.tail_next + g.members[q], t, blocks), "tail launch");
-                    launches += 2;
+                    launches += 1;
                     m.scene_totals[size_t(g.members[q]) * kSceneTotals + 5] += 1;
                 }
                 for (size_t k = 0; k < std::min(used, m.tail_streams.size()); ++k)

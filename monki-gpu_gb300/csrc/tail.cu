@@ -23,22 +23,16 @@ cudaError_t launch(const SceneView<T>& v, const Controls& c, const Divisors& dv,
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess && v.band_bytes)
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(v.band_bytes));
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, v.band_bytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTailBlock, v.band_bytes);
     if (e != cudaSuccess) return e;
-    // One resident wave per launch: the threads take entries until none is left. With
-    // `pending`, the events queued in buffer b first (they still need their scattering).
-    for (const bool first : {true, false}) {
-        if (first && !pending) continue;
-        e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
-        if (e != cudaSuccess) return e;
-        unsigned grid = unsigned(std::max(per_sm, 1) * sms);
-        if (max_blocks) grid = std::min(grid, max_blocks);
-        wf_tail<T, NMAT, PATHS, BACKWARD><<<grid, 256, v.band_bytes, stream>>>(
-            v, c, dv, P, banks, W, g, b, first, failure, counters, next);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    // One resident wave: the blocks take slots until none is left.
+    e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
+    if (e != cudaSuccess) return e;
+    unsigned grid = unsigned(std::max(per_sm, 1) * sms);
+    if (max_blocks) grid = std::min(grid, max_blocks);
+    wf_tail<T, NMAT, PATHS, BACKWARD><<<grid, kTailBlock, v.band_bytes, stream>>>(
+        v, c, dv, P, banks, W, g, b, pending, failure, counters, next);
+    return cudaGetLastError();
 }
 
 }  // namespace
