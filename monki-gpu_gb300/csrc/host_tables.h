@@ -245,7 +245,7 @@ struct Packed {
     std::vector<int> guides;
     size_t cells, zunit, zsum, ssalb_gas, albedo, tau_above, layer_beta, vprefix, run_lo, run_hi;
     size_t lut_f[kMaxSpecies], lut_cos[kMaxSpecies], lut_cdf[kMaxSpecies], guide[kMaxSpecies];
-    size_t lut_v[kMaxSpecies];
+    size_t lut_v[kMaxSpecies], node[kMaxSpecies];
     size_t band, band_count, extent;
     int uniform_top;
 };
@@ -389,6 +389,21 @@ Packed<T> pack(const Prepared& p, bool uniform_prefix, bool rectangles = true) {
                 v[k.lut_v[s] + 2 * i + 1] = T(l.f44[i]);
             }
         }
+        // A species that does not polarize has one table: its nodes carry everything the
+        // sampling and the phase function read, one vector load per node.
+        bool plain = true;
+        for (int i = 0; i < l.n && plain; ++i) {
+            const T f11 = T(l.f11[i]);
+            plain = f11 >= T(0) && T(l.f22[i]) == f11 && T(l.f33[i]) == f11 && T(l.f12[i]) == T(0);
+        }
+        k.node[s] = SIZE_MAX;
+        if (plain) {
+            k.node[s] = reserve(4 * size_t(l.n));
+            for (int i = 0; i < l.n; ++i) {
+                v[k.node[s] + 4 * i] = T(l.cos[i]); v[k.node[s] + 4 * i + 1] = T(l.cdf[i]);
+                v[k.node[s] + 4 * i + 2] = T(l.f11[i]);
+            }
+        }
         // Guide: largest i <= n - 2 with cdf[i] <= g / kGuide (at transport precision).
         k.guide[s] = k.guides.size();
         int i = 0;
@@ -440,6 +455,7 @@ SceneView<T> make_view(const Prepared& p, const Packed<T>& k, void* base) {
         s.lut_f[sp] = tv + k.lut_f[sp]; s.lut_cos[sp] = tv + k.lut_cos[sp]; s.lut_cdf[sp] = tv + k.lut_cdf[sp];
         s.guide[sp] = gv + k.guide[sp];
         s.lut_v[sp] = k.lut_v[sp] == SIZE_MAX ? nullptr : tv + k.lut_v[sp];
+        s.node[sp] = k.node[sp] == SIZE_MAX ? nullptr : tv + k.node[sp];
     }
     return s;
 }

@@ -17,6 +17,8 @@
 //   lut_f[4 * n]             {F11, F22, F33, F12} per scattering angle, per species
 //   lut_cos[n], lut_cdf[n]   ascending cosine grid and the bound-function CDF
 //   lut_v[2 * n]             {F34, F44} per scattering angle, per species (nmat 4 only)
+//   node[4 * n]              {cosine, CDF, F11, 0} per scattering angle, for plain species
+//                            (F22 = F33 = F11 >= 0 and F12 = 0 at every angle)
 //   guide[kGuide + 1]        CDF guide table: largest i with cdf[i] <= g / kGuide
 //   band[nx * ny * uniform_top]  extinction of every cell below the horizontally uniform
 //                            top (the only cells a cell walk visits), 16-byte aligned and
@@ -78,6 +80,7 @@ struct SceneView {
     const T* lut_cdf[kMaxSpecies];
     const int* guide[kMaxSpecies];
     const T* lut_v[kMaxSpecies];  // {F34, F44} per node (nmat 4), else null
+    const T* node[kMaxSpecies];   // plain species (F22 = F33 = F11, F12 = 0): their nodes, else null
     const T* band;          // extinction below the uniform top, i + nx * (j + ny * k)
     uint32_t band_bytes;    // padded size when staged in shared memory, else 0
     const uint32_t* extent; // equal-extinction rectangles of the band cells, or null
