@@ -77,11 +77,6 @@ template <typename T> __device__ __forceinline__ T fsign(T a, T b) { return sign
 template <typename T>
 struct Vec4 { T x, y, z, w; };
 
-// Keeps a value as the compiler sees it from being specialised by the branch it came from: the
-// arithmetic that follows is compiled, and its multiply-adds contracted, once for all of them.
-__device__ __forceinline__ void opaque(float& v) { asm volatile("" : "+f"(v)); }
-__device__ __forceinline__ void opaque(double& v) { asm volatile("" : "+d"(v)); }
-
 template <typename T>
 struct Phase { T f11, f22, f33, f12, f34, f44; };  // f34, f44 only for nmat 4
 
@@ -345,15 +340,15 @@ __device__ __forceinline__ T sample_cdf(const SceneView<T>& s, int sp, T u) {
 
 // Polarized rejection sampling: pdf F11 + F12 (Q cos 2 sigma + sign U sin 2 sigma) with
 // sign -1 forward and +1 backward. Rayleigh: uniform cosine with the F11(0 deg) bound;
-// particles: bound F11 + |F12| drawn from its CDF. Capped at 4096. `f` gets the scattering
-// matrix of the accepted direction, which the Stokes update needs too: with the vector-loaded
-// node records of plain species this took the box cloud from 145.1 to 127.6 ms per round of
-// 50,000 photons per column (30 x 20 columns; an arc cosine, two bracket walks and seven lerps
-// fewer per particle event, three lerps fewer per view of its peel-off).
+// particles: bound F11 + |F12| drawn from its CDF. Capped at 4096. The caller evaluates the
+// matrix of the accepted direction itself: handing it on saves an arc cosine and 0.5 % of a
+// box-cloud round (126.5 against 127.2 ms), but the Stokes update then rounds differently and
+// about one history in 10^9 scatters takes another path. The node records took the same round
+// (50,000 photons per column, 30 x 20 columns) from 145.1 to 129 ms.
 template <typename T, typename Stream>
 __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, int nmat, const T* st,
                                                  T cos_in, Stream& rng, T& cos_out, T& dphi,
-                                                 T& cos_sca, Phase<T>& f, T sign = T(-1)) {
+                                                 T& cos_sca, T sign = T(-1)) {
     const T pi = pi_v<T>();
     if (sp >= 0 && nmat < 4 && s.node[sp]) {
         // A plain species: its proposal is its phase function, so the first draw is always
@@ -369,8 +364,6 @@ __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, 
         const T cs = lut_lerp(u, a.y, b.y, a.x, b.x);
         const T sigma = T(2) * pi * T(rng.next()) - pi;
         rng.skip();
-        const T f11 = plain_f11<T>(node, n, lo, cs);
-        f = Phase<T>{f11, f11, f11, T(0), T(0), T(0)};
         cos_sca = cs;
         outgoing<T>(cos_in, cs, sigma, cos_out, dphi);
         return true;
@@ -380,7 +373,7 @@ __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, 
         T u1 = T(rng.next());
         T cs = sp < 0 ? T(2) * u1 - T(1) : sample_cdf<T>(s, sp, u1);
         T sigma = T(2) * pi * T(rng.next()) - pi;
-        f = phase<T>(s, sp, cs, nmat);
+        Phase<T> f = phase<T>(s, sp, cs, nmat);
         T pdf = f.f11;
         if (nmat > 1) {
             T s2, c2;

@@ -251,13 +251,13 @@ transport_kernel(SceneView<T> s, Controls ctl, TA* __restrict__ banks, TallyLayo
             }
             if (flag) break;
             T cos_out, dphi, cos_sca;
-            Phase<T> f;
-            if (!sample_direction<T>(s, sp, NMAT, st, c, rng, cos_out, dphi, cos_sca, f)) {
+            if (!sample_direction<T>(s, sp, NMAT, st, c, rng, cos_out, dphi, cos_sca)) {
                 flag = kSamplingCap; break;
             }
             const T phi_out = phi + dphi;
             {
                 Rot<T> r = NMAT > 1 ? rotation<T>(cos_sca, c, cos_out, phi, phi_out) : Rot<T>{T(1), T(0), T(1), T(0)};
+                Phase<T> f = phase<T>(s, sp, cos_sca, NMAT);
                 T ns[3];
                 scatter_stokes<T>(f, r, NMAT, st, ns);
                 const T s0 = ns[0];

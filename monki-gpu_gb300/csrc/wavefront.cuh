@@ -1200,7 +1200,6 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
         const T phi = dir0.w;
         T st[4] = {T(1), pol.x, pol.y, (NMAT > 3 && P.vee) ? P.vee[slot] : T(0)};
         T cos_out, dphi, cos_sca;
-        Phase<T> f;
         const bool guided = sp >= 0 && g.epsilon > T(0) && pos.w < g.cap;
         if (guided && T(rng.next()) < g.epsilon) {
             // Detector branch: a view, a cosine about it from the proposal, an azimuth.
@@ -1224,17 +1223,15 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
             T sp_, cp_;
             sincos(phi_out, &sp_, &cp_);
             cos_sca = fmin(T(1), fmax(T(-1), a0 * (cp_ * so) + b0 * (sp_ * so) + c0 * cos_out));
-            f = phase<T>(s, sp, cos_sca, NMAT);
         } else {
-            if (!sample_direction<T>(s, sp, NMAT, st, c0, rng, cos_out, dphi, cos_sca, f,
-                                     BACKWARD ? T(1) : T(-1))) {
+            if (!sample_direction<T>(s, sp, NMAT, st, c0, rng, cos_out, dphi, cos_sca, BACKWARD ? T(1) : T(-1))) {
                 atomicOr(failure, kSamplingCap);
                 return ended();
             }
             phi_out = phi + dphi;
         }
         const Rot<T> r = NMAT > 1 ? rotation<T>(cos_sca, c0, cos_out, phi, phi_out) : Rot<T>{T(1), T(0), T(1), T(0)};
-        opaque(f.f11); opaque(f.f22); opaque(f.f33); opaque(f.f12);
+        const Phase<T> f = phase<T>(s, sp, cos_sca, NMAT);
         T out[4] = {T(0), T(0), T(0), T(0)};
         if (BACKWARD) {
             // M = M P^T; the sampling vector is (M11, M12, -M13, M14).
