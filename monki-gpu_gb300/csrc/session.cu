@@ -274,7 +274,7 @@ void wave_iteration(Session& s, Recorder& rec, const SceneView<T>& v, Pool<T>& P
                static_cast<const T*>(s.scale), T(s.cfg.split)};
     // Fused: each event's scattering and its photon's next walk in one kernel (the events of
     // the previous iteration, peeled there). Unfused (scenes with layer paths by default):
-    // the walks in slot order, the peel-off, then the scatterings.
+    // the walks, the peel-off, then the scatterings.
     const bool fused = s.cfg.fused == 1 || (s.cfg.fused < 0 && !PATHS);
     if (fused) {
         if (v.backward)
@@ -284,7 +284,7 @@ void wave_iteration(Session& s, Recorder& rec, const SceneView<T>& v, Pool<T>& P
             rec.kernel(&wf_step<T, NMAT, PATHS, false>, slots_grid, block, v.band_bytes, v, c, dv, P, g, s.cfg.walk, cur,
                        s.failure, s.counters);
     } else {
-        rec.kernel(&wf_transit<T, PATHS>, slots_grid, block, v.band_bytes, v, c, dv, P, s.cfg.walk, out, s.failure,
+        rec.kernel(&wf_transit<T, PATHS>, slots_grid, block, v.band_bytes, v, c, dv, P, s.cfg.walk, cur, s.failure,
                    s.counters);
     }
     if (ev) rec.event(ev[1]);

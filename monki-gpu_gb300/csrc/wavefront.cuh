@@ -1073,6 +1073,18 @@ __device__ __forceinline__ void peel_phase(const SceneView<T>& s, const T* band,
     block_add<2>(totals, targets);
 }
 
+// True when a launch's block has no entry of the work lists `first` .. `last` of buffer b
+// (0-2 the event queues, 3 the paused walks, 4 the vacant slots): it ends before it stages the
+// band. Late in a round group most blocks of a launch are like that (box cloud, one round of
+// 50,000 photons per column: 128.6 -> 126.3 ms).
+template <typename T>
+__device__ __forceinline__ bool idle(const Pool<T>& P, uint32_t b, int first, int last) {
+    const uint32_t* c = P.counts + kListCounts * b;
+    uint32_t total = 0;
+    for (int q = first; q <= last; ++q) total += c[q];
+    return blockIdx.x * blockDim.x >= total;
+}
+
 // FP32: four blocks of 256 per SM (64 registers; +2.7 % on the layered cloud over three
 // blocks at 77 registers, the box cloud unchanged). FP64 stays at three: at 64 registers its
 // peel-off spills 200-400 bytes per thread.
@@ -1081,6 +1093,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3)
 wf_peel(SceneView<T> s, Controls ctl, Divisors dv, Pool<T> P, TA* __restrict__ banks, WaveTally L, uint32_t b,
         uint32_t* __restrict__ failure, unsigned long long* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char staged[];
+    if (idle(P, b, 0, 2)) return;
     const T* band = stage_band<T>(s, staged, failure);
     peel_phase<T, TA, NMAT, PATHS, BACKWARD>(s, band, ctl, dv, P, banks, L, b, failure, counters);
 }
@@ -1338,7 +1351,7 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
 // split copy or the next photon of the round group and walk it. One thread per list
 // entry: the lists hold at most one entry per slot.
 // ----------------------------------------------------------------------------------
-template <typename T, int NMAT, bool PATHS, bool BACKWARD, bool SMEM_HANDOFF = false>
+template <typename T, int NMAT, bool PATHS, bool BACKWARD, bool SMEM_HANDOFF = false, bool SCATTER = true>
 __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band, const Controls& ctl,
                                            const Divisors& dv, const Pool<T>& P, const Guide<T>& g, uint32_t walk,
                                            uint32_t cur, uint32_t* __restrict__ failure,
@@ -1362,7 +1375,7 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
     // room). 80-byte stride in FP32: the 16-byte accesses of a quarter warp fall in distinct
     // banks; 128 in FP64 for the 32-byte alignment of its records.
     constexpr int kHandStride = sizeof(T) == 4 ? 80 : 128;
-    __shared__ __align__(32) unsigned char hand[SMEM_HANDOFF ? 256 * kHandStride : 16];
+    __shared__ __align__(32) unsigned char hand[SCATTER && SMEM_HANDOFF ? 256 * kHandStride : 16];
     SlotState<T> local_state;
     SlotState<T>& state = SMEM_HANDOFF ? *reinterpret_cast<SlotState<T>*>(hand + threadIdx.x * kHandStride) : local_state;
     for (uint32_t e = block * blockDim.x + threadIdx.x; e < total; e += blocks * blockDim.x) {
@@ -1373,13 +1386,13 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
             slot = queue_entry(P.queue[cur], e, ns, ng, surface);
             if (slot >= P.capacity) { atomicOr(failure, kQueueCorrupt); continue; }
             // The new records go to the walk through the handoff (it may also leave the slot vacant).
-            scatter_event<T, NMAT, BACKWARD>(slot, surface, s, ctl, dv, P, g, failure, &state);
+            if (SCATTER) scatter_event<T, NMAT, BACKWARD>(slot, surface, s, ctl, dv, P, g, failure, &state);
         } else {
             slot = e < events + held ? P.paused[cur][e - events] : P.vacant[cur][e - events - held];
             if (slot >= P.capacity) { atomicOr(failure, kQueueCorrupt); continue; }
         }
         transit_slot<T, PATHS, true>(slot, s, band, ctl, dv, P, walk, may_claim, out, failure, scatters, visits,
-                                     scattered ? &state : nullptr);
+                                     SCATTER && scattered ? &state : nullptr);
     }
     const unsigned long long totals[2] = {scatters, visits};
     unsigned long long* const targets[2] = {counters + 0, counters + 1};
@@ -1391,30 +1404,26 @@ __global__ void __launch_bounds__(256, MONKI_STEP_BLOCKS)
 wf_step(SceneView<T> s, Controls ctl, Divisors dv, Pool<T> P, Guide<T> g, uint32_t walk, uint32_t cur,
         uint32_t* __restrict__ failure, unsigned long long* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char staged[];
+    if (idle(P, cur, 0, 4)) return;
     const T* band = stage_band<T>(s, staged, failure);
     step_phase<T, NMAT, PATHS, BACKWARD, true>(s, band, ctl, dv, P, g, walk, cur, failure, counters);
 }
 
 // The same iteration in two launches, for scenes with layer paths, whose walks and
 // scatterings together need more registers than one kernel has without spilling: the walks
-// of every slot in slot order (transit), then, after the peel-off, the scatterings of the
-// queued events (scatter). Both file slots in the work lists of buffer `out` like the step.
+// of every listed slot (transit; the queued events were scattered in the last iteration),
+// then, after the peel-off, the scatterings of the new events (scatter). Both work from the
+// lists like the step: a scan over every slot read four records of each, filled slot or not,
+// and took 105 us per launch at 2.4 M slots however few photons were left (layered cloud, two
+// rounds of 2,000 photons per column: 79.4 -> 65.8 ms with the lists).
 template <typename T, bool PATHS>
 __global__ void __launch_bounds__(256, 4)
-wf_transit(SceneView<T> s, Controls ctl, Divisors dv, Pool<T> P, uint32_t walk, uint32_t out,
+wf_transit(SceneView<T> s, Controls ctl, Divisors dv, Pool<T> P, uint32_t walk, uint32_t cur,
            uint32_t* __restrict__ failure, unsigned long long* __restrict__ counters) {
     extern __shared__ __align__(16) unsigned char staged[];
+    if (idle(P, cur, 0, 4)) return;
     const T* band = stage_band<T>(s, staged, failure);
-    uint64_t scatters = 0, visits = 0;
-    __shared__ uint32_t claims_open;
-    if (threadIdx.x == 0) claims_open = *reinterpret_cast<volatile uint32_t*>(P.counts + kClaimCount) < ctl.count;
-    __syncthreads();
-    const bool may_claim = claims_open != 0u;
-    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < P.capacity; slot += gridDim.x * blockDim.x)
-        transit_slot<T, PATHS, true>(slot, s, band, ctl, dv, P, walk, may_claim, out, failure, scatters, visits);
-    const unsigned long long totals[2] = {scatters, visits};
-    unsigned long long* const targets[2] = {counters + 0, counters + 1};
-    block_add<2>(totals, targets);
+    step_phase<T, 1, PATHS, false, true, false>(s, band, ctl, dv, P, Guide<T>{}, walk, cur, failure, counters);
 }
 
 template <typename T, int NMAT, bool BACKWARD>
