@@ -65,7 +65,11 @@ struct PhotonStream {
         ++lane;
         return (float(w >> 9) + 0.5f) * 0x1p-23f;
     }
-    __device__ __forceinline__ void skip() { next(); }
+    // The next three draws: one sampling attempt.
+    __device__ __forceinline__ void attempt(float (&u)[3]) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) u[q] = next();
+    }
 };
 
 template <typename T> __device__ __forceinline__ T fsign(T a, T b) { return signbit(b) ? -fabs(a) : fabs(a); }
@@ -350,29 +354,31 @@ __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, 
                                                  T cos_in, Stream& rng, T& cos_out, T& dphi,
                                                  T& cos_sca, T sign = T(-1)) {
     const T pi = pi_v<T>();
+    float u[3];
     if (sp >= 0 && nmat < 4 && s.node[sp]) {
         // A plain species: its proposal is its phase function, so the first draw is always
         // accepted (pdf and bound are both F11; the acceptance draw is spent all the same).
         const int n = s.lut_n[sp];
         const T* __restrict__ node = s.node[sp];
-        const T u = T(rng.next());
-        int g = int(u * T(kGuide));
+        rng.attempt(u);
+        const T u1 = T(u[0]);
+        int g = int(u1 * T(kGuide));
         g = g < 0 ? 0 : (g > kGuide ? kGuide : g);
         int lo = __ldg(s.guide[sp] + g);
         Vec4<T> a = load4(node + 4 * lo), b = load4(node + 4 * lo + 4);
-        while (lo < n - 2 && b.y < u) { ++lo; a = b; b = load4(node + 4 * lo + 4); }
-        const T cs = lut_lerp(u, a.y, b.y, a.x, b.x);
-        const T sigma = T(2) * pi * T(rng.next()) - pi;
-        rng.skip();
+        while (lo < n - 2 && b.y < u1) { ++lo; a = b; b = load4(node + 4 * lo + 4); }
+        const T cs = lut_lerp(u1, a.y, b.y, a.x, b.x);
+        const T sigma = T(2) * pi * T(u[1]) - pi;
         cos_sca = cs;
         outgoing<T>(cos_in, cs, sigma, cos_out, dphi);
         return true;
     }
     const T bound_gas = rayleigh<T>(T(1), s.depol, 1).f11;
     for (int attempt = 0; attempt < 4096; ++attempt) {
-        T u1 = T(rng.next());
+        rng.attempt(u);
+        T u1 = T(u[0]);
         T cs = sp < 0 ? T(2) * u1 - T(1) : sample_cdf<T>(s, sp, u1);
-        T sigma = T(2) * pi * T(rng.next()) - pi;
+        T sigma = T(2) * pi * T(u[1]) - pi;
         Phase<T> f = phase<T>(s, sp, cs, nmat);
         T pdf = f.f11;
         if (nmat > 1) {
@@ -381,7 +387,7 @@ __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, 
             pdf = f.f11 + f.f12 * (st[1] * c2 + sign * st[2] * s2);
         }
         T bound = sp < 0 ? bound_gas : f.f11 + fabs(f.f12);
-        if (T(rng.next()) * bound > pdf) continue;
+        if (T(u[2]) * bound > pdf) continue;
         cos_sca = cs;
         outgoing<T>(cos_in, cs, sigma, cos_out, dphi);
         return true;

@@ -263,6 +263,8 @@ __device__ __forceinline__ T band_beta(const SceneView<T>& s, const T* band, int
 }
 
 // A photon's Philox stream addressed by draw index: draw d is word d % 4 of block d / 4.
+__device__ __forceinline__ float draw_value(uint32_t w) { return (float(w >> 9) + 0.5f) * 0x1p-23f; }
+
 struct DrawStream {
     uint32_t photon, round, seed, draw, loaded, lineage;
     uint4 words;
@@ -271,18 +273,59 @@ struct DrawStream {
     __device__ __forceinline__ void init(uint32_t p, uint32_t r, uint32_t s, uint32_t d, uint32_t l = 0u) {
         photon = p; round = r; seed = s; draw = d; loaded = kNone; lineage = l;
     }
+    __device__ __forceinline__ uint4 block(uint32_t blk) const {
+        return philox4x32_10(make_uint4(photon, round, blk, lineage), make_uint2(seed, 0u));
+    }
     __device__ __forceinline__ float next() {
         const uint32_t blk = draw >> 2;
         if (blk != loaded) {
-            words = philox4x32_10(make_uint4(photon, round, blk, lineage), make_uint2(seed, 0u));
+            words = block(blk);
             loaded = blk;
         }
         const uint32_t lane = draw & 3u;
         const uint32_t w = lane == 0 ? words.x : lane == 1 ? words.y : lane == 2 ? words.z : words.w;
         ++draw;
-        return (float(w >> 9) + 0.5f) * 0x1p-23f;
+        return draw_value(w);
     }
-    __device__ __forceinline__ void skip() { ++draw; }
+};
+
+// The stream of a scattering, five draws at a time. The lanes of a warp stand at different
+// words of their blocks, so drawing one by one ran the ten Philox rounds at nearly every draw
+// for the quarter of the lanes that had come to a new block: a window makes both blocks that
+// five draws can touch, once for all lanes and side by side, and shifts them into place.
+// Guided box cloud, 32 rounds of 1,000 photons per column 71.5 -> 70.3 ms; clear sky, 32 rounds
+// of 2,000 46.0 -> 45.3 ms.
+struct DrawWindow {
+    DrawStream s;
+    uint32_t w[5];  // draws `start` .. start + 4
+    uint32_t start;
+    __device__ __forceinline__ void init(uint32_t p, uint32_t r, uint32_t seed, uint32_t d, uint32_t l) {
+        s.init(p, r, seed, d, l);
+        start = d - 8u;  // no window yet
+    }
+    __device__ __forceinline__ void open() {
+        start = s.draw;
+        const uint4 a = s.block(start >> 2), b = s.block((start >> 2) + 1u);
+        const bool one = start & 1u, two = start & 2u;
+        const uint32_t v0 = one ? a.y : a.x, v1 = one ? a.z : a.y, v2 = one ? a.w : a.z, v3 = one ? b.x : a.w,
+                       v4 = one ? b.y : b.x, v5 = one ? b.z : b.y, v6 = one ? b.w : b.z;
+        w[0] = two ? v2 : v0; w[1] = two ? v3 : v1; w[2] = two ? v4 : v2; w[3] = two ? v5 : v3; w[4] = two ? v6 : v4;
+    }
+    // The three draws of a sampling attempt: the first of a new window.
+    __device__ __forceinline__ void attempt(float (&u)[3]) {
+        open();
+#pragma unroll
+        for (int q = 0; q < 3; ++q) u[q] = draw_value(w[q]);
+        s.draw += 3u;
+    }
+    // A draw after an attempt: the window holds two, and the stream the others.
+    __device__ __forceinline__ float after() {
+        const uint32_t at = s.draw - start;
+        if (at > 4u) return s.next();
+        ++s.draw;
+        return draw_value(at == 4u ? w[4] : w[3]);
+    }
+    __device__ __forceinline__ float next() { return s.next(); }
 };
 
 // Reserve one entry of counters[key] per calling lane. Lanes that arrive together are
@@ -1170,7 +1213,7 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
         return false;
     }
     const uint32_t ro = dv.per_round.div(pid);
-    DrawStream rng;
+    DrawWindow rng;
     rng.init(pid - ro * ctl.per_round, ctl.first_round + ro, ctl.seed, meta.y, P.lineage ? P.lineage[slot] : 0u);
     const T a0 = dir0.x, b0 = dir0.y, c0 = dir0.z;
     T a, b, c, phi_out, q = T(0), u = T(0), v = T(0);
@@ -1187,9 +1230,13 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
     T roulette = g.roulette;
     if (g.scale) roulette *= __ldg(g.scale + ci + s.nx * (cj + s.ny * ck));
     if (surface) {
-        const T Pd = T(rng.next()), U = T(rng.next());
+        float u[3];
+        rng.attempt(u);
+        const T Pd = T(u[0]), U = T(u[1]);
+        rng.s.draw -= 1u;  // the third draw is spent by the roulette alone
         if (roulette > T(0) && pos.w < roulette) {
-            if (T(rng.next()) * roulette < pos.w) pos.w = roulette;
+            rng.s.draw += 1u;
+            if (T(u[2]) * roulette < pos.w) pos.w = roulette;
             else return ended();
         }
         const T mu = sqrt(Pd);
@@ -1287,7 +1334,7 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
         a = cpo * so; b = spo * so; c = cos_out;
         if (guided) pos.w *= ddis_factor<T, NMAT>(s, g, sp, cos_sca, s0, a, b, c);
         if (roulette > T(0) && pos.w < roulette) {
-            if (T(rng.next()) * roulette < pos.w) pos.w = roulette;
+            if (T(rng.after()) * roulette < pos.w) pos.w = roulette;
             else return ended();
         }
     }
@@ -1312,7 +1359,7 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
             for (int copy = 1; copy < n; ++copy) {
                 const size_t entry = size_t(slot) * kSplitStack + held + uint32_t(copy) - 1u;
                 SplitCopy<T>& cp = P.copies[entry];
-                cp.meta = make_uint4(pid, split_lineage(lineage, rng.draw, uint32_t(copy)), meta.z, meta.w);
+                cp.meta = make_uint4(pid, split_lineage(lineage, rng.s.draw, uint32_t(copy)), meta.z, meta.w);
                 cp.pos = pos;
                 cp.dir = dir_out;
                 cp.pol = pol_out;
@@ -1328,8 +1375,8 @@ __device__ __forceinline__ bool scatter_event(uint32_t slot, bool surface, const
 #pragma unroll
             for (int col = 0; col < NMAT; ++col) P.matrix[size_t(r * NMAT + col) * P.capacity + slot] = M[r][col];
     }
-    if (!surface) pol.z = -log(fmax(T(rng.next()), eps));
-    meta.y = rng.draw;
+    if (!surface) pol.z = -log(fmax(T(rng.after()), eps));
+    meta.y = rng.s.draw;
     const Quad<T> turned{a, b, c, phi_out};
     if (handoff) {
         *handoff = SlotState<T>{meta, pos, turned, pol};
