@@ -9,12 +9,14 @@
 //   W1[256 x 64], b1[256], W2[256 x 256], b2[256], W3[256 x 256], b3[256], w4[256], b4[1]
 //
 // Per layer l with input X (rows x K) and weights W (256 x K):
-//   forward   Z = X W^T + b (tcgen05, epilogue adds b, writes Z in BF16, H = GELU(Z), H^T;
+//   forward   Z = X W^T + b (tcgen05, epilogue adds b, writes Z in BF16, H = GELU(Z);
 //             the last layer's epilogue also forms the output y = H3 w4 + b4)
-//   backward  dW += dZ^T X (tcgen05 split-K over the rows, A = dZ^T, B = X^T)
+//   backward  dW += dZ^T X (tcgen05 split-K over the rows; dZ and X are read as they are
+//             stored, MN-major operands)
 //             dX' = (dZ W) * GELU'(Z_prev) (tcgen05, B = W^T, epilogue applies GELU' and
-//             adds the column sums of dX' to the previous layer's bias gradient)
-// so every operand is K-major and the transposed activations come from the epilogues.
+//             adds the column sums of dX' to the previous layer's bias gradient).
+// No transposed copies: writing them beside the activations and gradients took the epilogues
+// and half of the memory traffic of a step (300 steps at batch 65,536: 130.9 -> 113.1 ms).
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -55,29 +57,15 @@ void write_error(char* err, size_t n, const std::string& msg) {
 // Elementwise kernels.
 // ----------------------------------------------------------------------------------
 
-// Rows of FP32 features (gathered through idx when given) into the padded BF16 input and
-// its transpose; rows >= n and columns >= F are zero. Block: 256 threads over 64 rows; the
-// rows are read and X written row by row, then the tile is transposed in shared memory so
-// the XT rows are written as contiguous 128-byte segments too.
-constexpr int kPackRows = 64, kPackStride = kIn + 1;
+// n rows of FP32 features (gathered through idx when given) into the BF16 input, its columns
+// >= F zero. One thread per pair of columns.
 __global__ void __launch_bounds__(256)
-pack_input(const float* __restrict__ x, const uint32_t* __restrict__ idx, int n, int F, int R,
-           bf16* __restrict__ X, bf16* __restrict__ XT) {
-    __shared__ bf16 tile[kPackRows * kPackStride];
-    const int m0 = blockIdx.x * kPackRows;
-    for (int e = threadIdx.x; e < kPackRows * kIn; e += blockDim.x) {
-        const int q = e / kIn, c = e % kIn, m = m0 + q;
-        float v = 0.f;
-        if (m < n && c < F) v = x[size_t(idx ? idx[m] : uint32_t(m)) * F + c];
-        const bf16 b = __float2bfloat16(v);
-        tile[q * kPackStride + c] = b;
-        if (m < R) X[size_t(m) * kIn + c] = b;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < kPackRows * kIn; e += blockDim.x) {
-        const int c = e / kPackRows, q = e % kPackRows, m = m0 + q;
-        if (m < R) XT[size_t(c) * R + m] = tile[q * kPackStride + c];
-    }
+pack_input(const float* __restrict__ x, const uint32_t* __restrict__ idx, int n, int F, bf16* __restrict__ X) {
+    const int e = blockIdx.x * 256 + threadIdx.x, m = e / (kIn / 2), c = 2 * (e % (kIn / 2));
+    if (m >= n) return;
+    const float* row = x + size_t(idx ? idx[m] : uint32_t(m)) * F;
+    const float v[2] = {c < F ? row[c] : 0.f, c + 1 < F ? row[c + 1] : 0.f};
+    *reinterpret_cast<__nv_bfloat162*>(X + size_t(m) * kIn + c) = __floats2bfloat162_rn(v[0], v[1]);
 }
 
 __global__ void gather_targets(const float* __restrict__ t, const float* __restrict__ w, const uint32_t* __restrict__ idx,
@@ -112,17 +100,13 @@ __global__ void loss_grad(const float* __restrict__ y, const float* __restrict__
     if ((threadIdx.x & 31) == 0 && part != 0.f) atomicAdd(loss, part);
 }
 
-// Output layer backward: dw4 += dy^T H3, db4 += sum dy, dZ3 = dy w4^T * GELU'(Z3) in BF16,
-// its transpose and db3 += the column sums of dZ3. Block: 256 threads (one per hidden unit)
-// over a slab of 64 rows; the slab's dZ3 is staged in shared memory (odd row stride, so the
-// column reads are free of bank conflicts) and each warp then writes 32 rows of the
-// transpose as 128-byte segments. Rows from `rows` to the slab's end are written as zeros.
-constexpr int kSlab = 64, kSlabStride = kHidden + 1;
+// Output layer backward: dw4 += dy^T H3, db4 += sum dy, dZ3 = dy w4^T * GELU'(Z3) in BF16 and
+// db3 += the column sums of dZ3. Block: 256 threads (one per hidden unit) over a slab of 64
+// rows.
+constexpr int kSlab = 64;
 __global__ void __launch_bounds__(kHidden)
 head_backward(const float* __restrict__ dy, const bf16* __restrict__ H, const float* __restrict__ w4,
-              const bf16* __restrict__ Z, int rows, int R, float* __restrict__ grads, bf16* __restrict__ G,
-              bf16* __restrict__ GT) {
-    __shared__ bf16 tile[kSlab * kSlabStride];
+              const bf16* __restrict__ Z, int rows, float* __restrict__ grads, bf16* __restrict__ G) {
     const int n = threadIdx.x;
     const int m0 = blockIdx.x * kSlab;
     float acc = 0.f, bias = 0.f, column = 0.f;
@@ -143,57 +127,55 @@ head_backward(const float* __restrict__ dy, const bf16* __restrict__ H, const fl
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int m = m0 + q0 + u;
-            bf16 g = __float2bfloat16(0.f);
             if (m < rows) {
                 acc += d[u] * __bfloat162float(h[u]);
                 bias += d[u];
-                g = __float2bfloat16(d[u] * wn * umma::gelu_grad(__bfloat162float(z[u])));
+                const bf16 g = __float2bfloat16(d[u] * wn * umma::gelu_grad(__bfloat162float(z[u])));
                 G[size_t(m) * kHidden + n] = g;
                 column += __bfloat162float(g);
             }
-            tile[(q0 + u) * kSlabStride + n] = g;
         }
     }
     atomicAdd(grads + ow4 + n, acc);
     atomicAdd(grads + ob3 + n, column);
     if (n == 0) atomicAdd(grads + ob4, bias);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m = m0 + 2 * lane;
-    for (int c = warp; c < kHidden; c += kHidden / 32) {
-        __nv_bfloat162 pair;
-        pair.x = tile[(2 * lane) * kSlabStride + c];
-        pair.y = tile[(2 * lane + 1) * kSlabStride + c];
-        bf16* dst = GT + size_t(c) * R + m;
-        if (m + 1 < R) *reinterpret_cast<__nv_bfloat162*>(dst) = pair;
-        else if (m < R) dst[0] = pair.x;
+}
+
+// BF16 working copies of the weights and the transposes the backward pass needs.
+struct Copies { bf16 *W1, *W2, *W3, *W2T, *W3T; };
+__device__ __forceinline__ void copy_weight(const Copies& k, size_t e, float p) {
+    const bf16 w = __float2bfloat16(p);
+    if (e < kW1) {
+        k.W1[e] = w;
+    } else if (e >= oW2 && e < oW2 + kW2) {
+        const size_t q = e - oW2;
+        k.W2[q] = w;
+        k.W2T[q % kHidden * kHidden + q / kHidden] = w;
+    } else if (e >= oW3 && e < oW3 + kW2) {
+        const size_t q = e - oW3;
+        k.W3[q] = w;
+        k.W3T[q % kHidden * kHidden + q / kHidden] = w;
     }
 }
 
+// One Adam step; the new weights' working copies are written with them.
 __global__ void adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1, float* __restrict__ m2,
-                     size_t count, float lr, float c1, float c2) {
+                     size_t count, float lr, float c1, float c2, Copies k) {
     for (size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < count; e += size_t(gridDim.x) * blockDim.x) {
         const float gi = g[e];
         const float a = 0.9f * m1[e] + 0.1f * gi;
         const float b = 0.999f * m2[e] + 0.001f * gi * gi;
         m1[e] = a;
         m2[e] = b;
-        p[e] -= lr * (a * c1) / (sqrtf(b * c2) + 1e-8f);
+        const float next = p[e] - lr * (a * c1) / (sqrtf(b * c2) + 1e-8f);
+        p[e] = next;
+        copy_weight(k, e, next);
     }
 }
 
-// BF16 working copies of the weights and the transposes the backward pass needs.
-__global__ void refresh(const float* __restrict__ p, bf16* __restrict__ W1, bf16* __restrict__ W2, bf16* __restrict__ W3,
-                        bf16* __restrict__ W2T, bf16* __restrict__ W3T) {
-    for (size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < kW2; e += size_t(gridDim.x) * blockDim.x) {
-        const size_t r = e / kHidden, c = e % kHidden;
-        if (e < kW1) W1[e] = __float2bfloat16(p[oW1 + e]);
-        const bf16 w2 = __float2bfloat16(p[oW2 + e]), w3 = __float2bfloat16(p[oW3 + e]);
-        W2[e] = w2;
-        W3[e] = w3;
-        W2T[c * kHidden + r] = w2;
-        W3T[c * kHidden + r] = w3;
-    }
+__global__ void refresh(const float* __restrict__ p, size_t count, Copies k) {
+    for (size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < count; e += size_t(gridDim.x) * blockDim.x)
+        copy_weight(k, e, p[e]);
 }
 
 // ----------------------------------------------------------------------------------
@@ -204,8 +186,7 @@ struct Net {
     cudaStream_t stream = nullptr;
     float *params = nullptr, *grads = nullptr, *m1 = nullptr, *m2 = nullptr;
     bf16 *W1 = nullptr, *W2 = nullptr, *W3 = nullptr, *W2T = nullptr, *W3T = nullptr;
-    bf16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *H1T = nullptr, *H2T = nullptr;
-    bf16 *G3 = nullptr, *G3T = nullptr, *G2 = nullptr, *G2T = nullptr, *G1 = nullptr, *G1T = nullptr;
+    bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *G3 = nullptr, *G2 = nullptr, *G1 = nullptr;
     bf16 *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr;  // pre-activations
     float *y = nullptr, *dy = nullptr, *tb = nullptr, *wb = nullptr;
     float* loss = nullptr;
@@ -216,6 +197,7 @@ struct Net {
     uint32_t step = 0, seed = 0;
     std::vector<void*> owned;
 
+    Copies copies() const { return Copies{W1, W2, W3, W2T, W3T}; }
     template <typename P>
     P* alloc(size_t count) {
         void* p = nullptr;
@@ -237,10 +219,12 @@ bool g_attr_done[64] = {};
 void configure(int device) {
     std::lock_guard<std::mutex> guard(g_attr_lock);
     if (device < 0 || device >= 64 || g_attr_done[device]) return;
-    check(cudaFuncSetAttribute(umma::gemm<umma::kStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kBackward>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kAccumulate>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    check(cudaFuncSetAttribute(umma::gemm<umma::kStore, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kForward, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kBackward, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kAccumulate, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               umma::smem_bytes_of<umma::kAccumulate>()), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kAccumulate, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                umma::smem_bytes_of<umma::kAccumulate>()), "attr");
     g_attr_done[device] = true;
 }
@@ -264,15 +248,15 @@ EncodeTiled encoder() {
     return fn;
 }
 
-// Tensor map of a K-major BF16 matrix (rows x k_extent, row stride ld elements) read in
-// tiles of 64 K-elements (128 bytes, the swizzle width) x box_rows rows; reads outside the
-// matrix return zeros.
-CUtensorMap tile_map(const bf16* base, int rows, int k_extent, int ld, int box_rows) {
-    if ((reinterpret_cast<uintptr_t>(base) & 15) || (size_t(ld) * sizeof(bf16)) % 16 || k_extent % umma::kBlockK ||
+// Tensor map of a row-major BF16 matrix (rows x columns, row stride ld elements) read in tiles
+// of 64 columns (128 bytes, the swizzle width) x box_rows rows; reads outside the matrix return
+// zeros.
+CUtensorMap tile_map(const bf16* base, int rows, int columns, int ld, int box_rows) {
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || (size_t(ld) * sizeof(bf16)) % 16 || columns % umma::kBlockK ||
         box_rows < 1 || box_rows > 256)
         throw std::runtime_error("operand outside the tensor-map tiling");
     CUtensorMap map{};
-    const cuuint64_t dims[2] = {cuuint64_t(k_extent), cuuint64_t(rows)};
+    const cuuint64_t dims[2] = {cuuint64_t(columns), cuuint64_t(rows)};
     const cuuint64_t strides[1] = {cuuint64_t(ld) * sizeof(bf16)};
     const cuuint32_t box[2] = {cuuint32_t(umma::kBlockK), cuuint32_t(box_rows)};
     const cuuint32_t element[2] = {1, 1};
@@ -283,7 +267,8 @@ CUtensorMap tile_map(const bf16* base, int rows, int k_extent, int ld, int box_r
     return map;
 }
 
-// One GEMM: operands (K-major, row strides lda / ldb) and the epilogue's parameters.
+// One GEMM: operands (K-major, row strides lda / ldb; MN-major, row strides lda / ldb of the
+// row-major matrices whose rows are contracted) and the epilogue's parameters.
 struct Gemm {
     const bf16* A;
     int lda;
@@ -292,15 +277,19 @@ struct Gemm {
     umma::Params p;
 };
 
-template <int EPI>
-void gemm(const Gemm& g, int splits, cudaStream_t stream) {
+// `rows` (MN-major): the valid rows; the tensor maps return zeros for those up to K.
+template <int EPI, bool MN = false>
+void gemm(const Gemm& g, int splits, cudaStream_t stream, int rows = 0) {
     const umma::Params& p = g.p;
-    if (p.K % umma::kBlockK || p.k_chunk % umma::kBlockK || p.N % 16 || p.N < 16 || p.N > 256 || p.rows_a < 1)
+    if (p.K % umma::kBlockK || p.k_chunk % umma::kBlockK || p.N % 16 || p.N < 16 || p.N > 256 || p.rows_a < 1 ||
+        (MN && (p.N % 64 || p.rows_a % umma::kBlockM || rows < 1)))
         throw std::runtime_error("GEMM shape outside the kernel's tiling");
-    const CUtensorMap map_a = tile_map(g.A, p.rows_a, p.K, g.lda, umma::kBlockM);
-    const CUtensorMap map_b = tile_map(g.B, p.N, p.K, g.ldb, p.N);
+    const CUtensorMap map_a = MN ? tile_map(g.A, rows, p.rows_a, g.lda, umma::kBlockK)
+                                 : tile_map(g.A, p.rows_a, p.K, g.lda, umma::kBlockM);
+    const CUtensorMap map_b = MN ? tile_map(g.B, rows, p.N, g.ldb, umma::kBlockK)
+                                 : tile_map(g.B, p.N, p.K, g.ldb, p.N);
     dim3 grid((p.rows_a + umma::kBlockM - 1) / umma::kBlockM, splits);
-    umma::gemm<EPI><<<grid, umma::kThreads, umma::smem_bytes_of<EPI>(), stream>>>(map_a, map_b, p);
+    umma::gemm<EPI, MN><<<grid, umma::kThreads, umma::smem_bytes_of<EPI>(), stream>>>(map_a, map_b, p);
     check(cudaGetLastError(), "gemm launch");
 }
 
@@ -311,66 +300,55 @@ Gemm params_for(const bf16* A, const bf16* B, int rows, int N, int K, uint32_t* 
     return g;
 }
 
-// Zero the columns [rows, rows rounded up to 64) of a transposed (height x R) matrix: the
-// split-K weight-gradient GEMMs read whole 64-column slices.
-void clear_tail(bf16* T, int rows, int R, int height, cudaStream_t stream) {
-    const int end = std::min(R, (rows + 63) / 64 * 64);
-    if (end > rows)
-        check(cudaMemset2DAsync(T + rows, size_t(R) * sizeof(bf16), 0, size_t(end - rows) * sizeof(bf16), size_t(height), stream),
-              "memset(tail)");
+void pack_rows(Net& n, const float* x, const uint32_t* idx, int rows) {
+    pack_input<<<(rows * (kIn / 2) + 255) / 256, 256, 0, n.stream>>>(x, idx, rows, n.features, n.X);
+    check(cudaGetLastError(), "pack launch");
 }
 
 // Forward pass of the first `rows` rows (<= R) of the packed input.
 void forward(Net& n, int rows) {
-    const int R = n.R;
     Gemm g = params_for(n.X, n.W1, rows, kHidden, kIn, n.failure);
-    g.p.Z = n.Z1; g.p.bias = n.params + ob1; g.p.H = n.H1; g.p.HT = n.H1T; g.p.rows_ht = R;
+    g.p.Z = n.Z1; g.p.bias = n.params + ob1; g.p.H = n.H1;
     gemm<umma::kForward>(g, 1, n.stream);
     g = params_for(n.H1, n.W2, rows, kHidden, kHidden, n.failure);
-    g.p.Z = n.Z2; g.p.bias = n.params + ob2; g.p.H = n.H2; g.p.HT = n.H2T; g.p.rows_ht = R;
+    g.p.Z = n.Z2; g.p.bias = n.params + ob2; g.p.H = n.H2;
     gemm<umma::kForward>(g, 1, n.stream);
     g = params_for(n.H2, n.W3, rows, kHidden, kHidden, n.failure);
-    g.p.Z = n.Z3; g.p.bias = n.params + ob3; g.p.H = n.H3; g.p.HT = nullptr; g.p.rows_ht = R;
+    g.p.Z = n.Z3; g.p.bias = n.params + ob3; g.p.H = n.H3;
     // The output layer rides on this epilogue: y = H3 w4 + b4.
     g.p.head_w = n.params + ow4; g.p.head_b = n.params + ob4; g.p.head_y = n.y;
     gemm<umma::kForward>(g, 1, n.stream);
-    clear_tail(n.H1T, rows, R, kHidden, n.stream);
-    clear_tail(n.H2T, rows, R, kHidden, n.stream);
 }
 
 // Loss and gradients of the first `rows` rows against tb / wb (gradients accumulate into
 // n.grads, which the caller clears).
 void backward(Net& n, int rows, float inv_weight, float* loss) {
-    const int R = n.R;
     loss_grad<<<256, 256, 0, n.stream>>>(n.y, n.tb, n.wb, rows, inv_weight, n.dy, loss);
-    head_backward<<<(rows + 63) / 64, kHidden, 0, n.stream>>>(n.dy, n.H3, n.params + ow4, n.Z3, rows, R, n.grads,
-                                                              n.G3, n.G3T);
+    head_backward<<<(rows + kSlab - 1) / kSlab, kHidden, 0, n.stream>>>(n.dy, n.H3, n.params + ow4, n.Z3, rows, n.grads, n.G3);
     check(cudaGetLastError(), "head backward launch");
     // Split-K over the rows for the weight gradients: 64-row multiples, slices of 1,024 rows
     // (at batch 65,536 two row tiles x 64 slices = 128 CTAs, each adding one partial).
     const int chunk = 1024, K = (rows + 63) / 64 * 64, splits = (K + chunk - 1) / chunk;
-    Gemm g = params_for(n.G3T, n.H2T, kHidden, kHidden, K, n.failure);
-    g.lda = R; g.ldb = R; g.p.k_chunk = chunk; g.p.C = n.grads + oW3;
-    gemm<umma::kAccumulate>(g, splits, n.stream);
-    g = params_for(n.G3, n.W3T, rows, kHidden, kHidden, n.failure);
-    g.p.zprev = n.Z2; g.p.H = n.G2; g.p.HT = n.G2T; g.p.rows_ht = R; g.p.bias_grad = n.grads + ob2;
-    gemm<umma::kBackward>(g, 1, n.stream);
-    clear_tail(n.G2T, rows, R, kHidden, n.stream);
-    g = params_for(n.G2T, n.H1T, kHidden, kHidden, K, n.failure);
-    g.lda = R; g.ldb = R; g.p.k_chunk = chunk; g.p.C = n.grads + oW2;
-    gemm<umma::kAccumulate>(g, splits, n.stream);
-    g = params_for(n.G2, n.W2T, rows, kHidden, kHidden, n.failure);
-    g.p.zprev = n.Z1; g.p.H = n.G1; g.p.HT = n.G1T; g.p.rows_ht = R; g.p.bias_grad = n.grads + ob1;
-    gemm<umma::kBackward>(g, 1, n.stream);
-    clear_tail(n.G1T, rows, R, kHidden, n.stream);
-    g = params_for(n.G1T, n.XT, kHidden, kIn, K, n.failure);
-    g.lda = R; g.ldb = R; g.p.k_chunk = chunk; g.p.C = n.grads + oW1;
-    gemm<umma::kAccumulate>(g, splits, n.stream);
+    auto weight_gradient = [&](const bf16* dZ, const bf16* in, int width, float* out) {
+        Gemm g = params_for(dZ, in, kHidden, width, K, n.failure);
+        g.lda = kHidden; g.ldb = width; g.p.k_chunk = chunk; g.p.C = out;
+        gemm<umma::kAccumulate, true>(g, splits, n.stream, rows);
+    };
+    auto input_gradient = [&](const bf16* dZ, const bf16* WT, const bf16* zprev, bf16* out, float* bias_grad) {
+        Gemm g = params_for(dZ, WT, rows, kHidden, kHidden, n.failure);
+        g.p.zprev = zprev; g.p.H = out; g.p.bias_grad = bias_grad;
+        gemm<umma::kBackward>(g, 1, n.stream);
+    };
+    weight_gradient(n.G3, n.H2, kHidden, n.grads + oW3);
+    input_gradient(n.G3, n.W3T, n.Z2, n.G2, n.grads + ob2);
+    weight_gradient(n.G2, n.H1, kHidden, n.grads + oW2);
+    input_gradient(n.G2, n.W2T, n.Z1, n.G1, n.grads + ob1);
+    weight_gradient(n.G1, n.X, kIn, n.grads + oW1);
     check(cudaGetLastError(), "backward launch");
 }
 
 void refresh_weights(Net& n) {
-    refresh<<<256, 256, 0, n.stream>>>(n.params, n.W1, n.W2, n.W3, n.W2T, n.W3T);
+    refresh<<<592, 256, 0, n.stream>>>(n.params, kParams, n.copies());
     check(cudaGetLastError(), "refresh launch");
 }
 
@@ -416,8 +394,8 @@ void* monki_mlp_create(uint32_t device, uint32_t features, uint32_t rows, uint32
         n->m1 = n->alloc<float>(kParams); n->m2 = n->alloc<float>(kParams);
         n->W1 = n->alloc<bf16>(kW1); n->W2 = n->alloc<bf16>(kW2); n->W3 = n->alloc<bf16>(kW2);
         n->W2T = n->alloc<bf16>(kW2); n->W3T = n->alloc<bf16>(kW2);
-        n->X = n->alloc<bf16>(R * kIn); n->XT = n->alloc<bf16>(R * kIn);
-        for (bf16** b : {&n->H1, &n->H2, &n->H3, &n->H1T, &n->H2T, &n->G3, &n->G3T, &n->G2, &n->G2T, &n->G1, &n->G1T})
+        n->X = n->alloc<bf16>(R * kIn);
+        for (bf16** b : {&n->H1, &n->H2, &n->H3, &n->G3, &n->G2, &n->G1})
             *b = n->alloc<bf16>(R * H);
         n->Z1 = n->alloc<bf16>(R * H); n->Z2 = n->alloc<bf16>(R * H); n->Z3 = n->alloc<bf16>(R * H);
         n->y = n->alloc<float>(R); n->dy = n->alloc<float>(R); n->tb = n->alloc<float>(R); n->wb = n->alloc<float>(R);
@@ -428,9 +406,6 @@ void* monki_mlp_create(uint32_t device, uint32_t features, uint32_t rows, uint32
         check(cudaMemset(n->m1, 0, kParams * sizeof(float)), "memset");
         check(cudaMemset(n->m2, 0, kParams * sizeof(float)), "memset");
         check(cudaMemset(n->failure, 0, sizeof(uint32_t)), "memset");
-        // Transposed activations are read in 64-row slices; the padding rows stay zero.
-        for (bf16* b : {n->XT, n->H1T, n->H2T, n->G3T, n->G2T, n->G1T})
-            check(cudaMemset(b, 0, R * (b == n->XT ? size_t(kIn) : H) * sizeof(bf16)), "memset");
         refresh_weights(*n);
         check(cudaStreamSynchronize(n->stream), "create");
         return n;
@@ -488,7 +463,7 @@ int monki_mlp_forward(void* handle, const float* x, uint32_t rows, float* y, cha
                 const int m = int(std::min<uint32_t>(uint32_t(n->R), rows - r0));
                 check(cudaMemcpyAsync(dx, x + size_t(r0) * n->features, size_t(m) * n->features * sizeof(float),
                                       cudaMemcpyHostToDevice, n->stream), "upload");
-                pack_input<<<(n->R + kPackRows - 1) / kPackRows, 256, 0, n->stream>>>(dx, nullptr, m, n->features, n->R, n->X, n->XT);
+                pack_rows(*n, dx, nullptr, m);
                 forward(*n, m);
                 check(cudaMemcpyAsync(y + r0, n->y, size_t(m) * sizeof(float), cudaMemcpyDeviceToHost, n->stream), "download");
                 check_failure(*n);
@@ -523,7 +498,7 @@ int monki_mlp_gradients(void* handle, const float* x, const float* target, const
         check(cudaMemcpyAsync(dx, x, size_t(rows) * n->features * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
         check(cudaMemcpyAsync(dt, target, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
         check(cudaMemcpyAsync(dw, weight, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
-        pack_input<<<(n->R + kPackRows - 1) / kPackRows, 256, 0, n->stream>>>(dx, nullptr, int(rows), n->features, n->R, n->X, n->XT);
+        pack_rows(*n, dx, nullptr, int(rows));
         gather_targets<<<256, 256, 0, n->stream>>>(dt, dw, nullptr, int(rows), n->R, n->tb, n->wb);
         check(cudaMemsetAsync(n->grads, 0, kParams * sizeof(float), n->stream), "memset");
         check(cudaMemsetAsync(n->loss, 0, sizeof(float), n->stream), "memset");
@@ -582,7 +557,7 @@ int monki_mlp_train(void* handle, uint32_t steps, uint32_t batch, float lr, floa
             for (uint32_t s = 0; s < steps; ++s) {
                 const uint32_t t = ++n->step;
                 sample_indices<<<(batch + 255) / 256, 256, 0, n->stream>>>(t, n->seed, int(batch), n->data_n, n->idx);
-                pack_input<<<(n->R + kPackRows - 1) / kPackRows, 256, 0, n->stream>>>(n->data_x, n->idx, int(batch), n->features, n->R, n->X, n->XT);
+                pack_rows(*n, n->data_x, n->idx, int(batch));
                 gather_targets<<<256, 256, 0, n->stream>>>(n->data_t, n->data_w, n->idx, int(batch), n->R, n->tb, n->wb);
                 check(cudaMemsetAsync(n->grads, 0, kParams * sizeof(float), n->stream), "memset");
                 forward(*n, int(batch));
@@ -591,8 +566,7 @@ int monki_mlp_train(void* handle, uint32_t steps, uint32_t batch, float lr, floa
                 // depend on the batch.
                 backward(*n, int(batch), 1.0f / float(batch), dloss + s);
                 const float c1 = 1.f / (1.f - std::pow(0.9f, float(t))), c2 = 1.f / (1.f - std::pow(0.999f, float(t)));
-                adam<<<592, 256, 0, n->stream>>>(n->params, n->grads, n->m1, n->m2, kParams, lr, c1, c2);
-                refresh_weights(*n);
+                adam<<<592, 256, 0, n->stream>>>(n->params, n->grads, n->m1, n->m2, kParams, lr, c1, c2, n->copies());
                 check(cudaGetLastError(), "train launch");
             }
             check(cudaMemcpyAsync(host_loss.data(), dloss, steps * sizeof(float), cudaMemcpyDeviceToHost, n->stream), "download");

@@ -11,15 +11,15 @@
 //             load; the last commit also arrives on the "done" mbarrier;
 //   epilogue  (all eight warps) after "done": TMEM lanes 32 (w % 4) .. + 31, every other
 //             32-column chunk from 32 (w / 4); bias, GELU or GELU', FP32 / BF16 stores, and
-//             transposed BF16 stores staged through shared memory so that each thread
-//             writes 64 contiguous bytes of a transposed row (and, in the backward
-//             epilogue, adds that row's 32 values to the column's bias gradient).
+//             in the backward epilogue the column sums of each warp's 32 rows (a butterfly of
+//             shuffles) are added to the bias gradient.
 //
 // Tile: 128 rows of C per CTA (the MMA's M), all N <= 256 columns (one MMA covers them),
 // K in steps of 64 (one 128-byte swizzle row of BF16). The K range of a CTA is blockIdx.y's
-// slice (split-K for the weight gradients, summed by float4 atomics). Every mbarrier wait is
-// bounded: a wait that gives up sets failure bit 1, the CTA skips its stores and still
-// releases its TMEM.
+// slice (split-K for the weight gradients, summed by float4 atomics; their operands are the
+// row-major gradients and activations themselves, contracted over the rows: MN-major). Every
+// mbarrier wait is bounded: a wait that gives up sets failure bit 1, the CTA skips its stores
+// and still releases its TMEM.
 //
 // Shared-memory operand layout (K-major, SWIZZLE_128B, what the TMA writes with
 // CU_TENSOR_MAP_SWIZZLE_128B): row r of a tile occupies bytes [128 r, 128 r + 128); its
@@ -45,12 +45,11 @@ constexpr uint32_t kStage = kSmemA + kSmemB;         // 48 KB, 1024-byte multipl
 // their TMEM allocations (256 columns each of the SM's 512) never wait on each other.
 constexpr uint32_t kSmemBytes = 100u * 1024u;
 constexpr uint32_t kWaitLimit = 1u << 24;          // mbarrier polls before giving up
-constexpr uint32_t kTransposeStride = 80;          // bytes per staged transposed row (32 BF16 + padding)
 
 enum Epilogue : int {
     kStore = 0,      // C (fp32) = acc
-    kForward = 1,    // Z (bf16) = acc + bias; H (bf16) = GELU(Z); H^T (bf16)
-    kBackward = 2,   // G = acc * GELU'(Zprev); G (bf16), G^T (bf16), column sums of G
+    kForward = 1,    // Z (bf16) = acc + bias; H (bf16) = GELU(Z)
+    kBackward = 2,   // G = acc * GELU'(Zprev); G (bf16), column sums of G
     kAccumulate = 3, // C (fp32) += acc (split-K partial, atomics)
 };
 
@@ -69,10 +68,8 @@ struct Params {
     __nv_bfloat16* Z;         // kForward: rows_a x N pre-activations (BF16)
     const float* bias;        // kForward: N
     const __nv_bfloat16* zprev;  // kBackward: rows_a x N pre-activations (BF16)
-    float* bias_grad;         // kBackward: N column sums of G are added here (needs HT), or null
+    float* bias_grad;         // kBackward: N column sums of G are added here, or null
     __nv_bfloat16* H;         // kForward / kBackward: rows_a x N
-    __nv_bfloat16* HT;        // kForward / kBackward: N x rows_ht (transposed), or null
-    int rows_ht;              // row stride of HT (>= rows_a, a multiple of 8)
     // kForward, optional: a linear output layer on the BF16 activations, y = H head_w +
     // head_b[0] per row (head_w: N values), written to head_y (rows_a values).
     const float* head_w;
@@ -96,9 +93,24 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return d;
 }
 
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major.
-__host__ __device__ constexpr uint32_t instr_desc(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
+// The same for an MN-major operand, a matrix whose contracted dimension runs over its rows:
+// blocks of 64 columns (one 128-byte swizzle row each) x 64 rows, 8 KB apart (leading byte
+// offset), eight rows of a block 1024 bytes (stride byte offset). 16 rows on, the next K = 16.
+constexpr uint32_t kBlockMN = 64 * kBlockK * 2;
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr) {
+    uint64_t d = 0;
+    d |= uint64_t((addr & 0x3FFFFu) >> 4);
+    d |= uint64_t(kBlockMN >> 4) << 16;
+    d |= uint64_t(1024u >> 4) << 32;
+    d |= uint64_t(1) << 46;
+    d |= uint64_t(2) << 61;
+    return d;
+}
+
+// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major or both
+// MN-major.
+__host__ __device__ constexpr uint32_t instr_desc(int m, int n, bool mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn ? 3u << 15 : 0u) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }
 
 __device__ __forceinline__ float gelu(float z) {
@@ -129,7 +141,7 @@ __device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, i
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 
-template <int EPI>
+template <int EPI, bool MN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, Params p) {
     extern __shared__ __align__(1024) unsigned char raw[];
@@ -185,13 +197,18 @@ gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensor
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(stage_bytes) : "memory");
             const uint32_t tile_a = smem_u32(base + s * kStage), tile_b = tile_a + kSmemA;
             const int k0 = k_begin + step * kBlockK;
-            tma_load(tile_a, &map_a, k0, row0, full);
-            tma_load(tile_b, &map_b, k0, 0, full);
+            if (MN) {
+                for (int c = 0; c < kBlockM; c += 64) tma_load(tile_a + uint32_t(c / 64) * kBlockMN, &map_a, row0 + c, k0, full);
+                for (int c = 0; c < N; c += 64) tma_load(tile_b + uint32_t(c / 64) * kBlockMN, &map_b, c, k0, full);
+            } else {
+                tma_load(tile_a, &map_a, k0, row0, full);
+                tma_load(tile_b, &map_b, k0, 0, full);
+            }
             issued = step + 1;
         }
     } else if (threadIdx.x == 32 && steps > 0) {
         // MMA issuer.
-        const uint32_t idesc = instr_desc(kBlockM, N);
+        const uint32_t idesc = instr_desc(kBlockM, N, MN);
         for (int step = 0; step < steps; ++step) {
             const int s = step % kRing, round = step / kRing;
             if (!wait_parity(smem_u32(&full_bar[s]), uint32_t(round) & 1u)) {
@@ -203,7 +220,8 @@ gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensor
             const uint32_t a_addr = smem_u32(base + s * kStage), b_addr = a_addr + kSmemA;
 #pragma unroll
             for (int kk = 0; kk < kBlockK / 16; ++kk) {
-                const uint64_t da = smem_desc(a_addr + kk * 32), db = smem_desc(b_addr + kk * 32);
+                const uint64_t da = MN ? smem_desc_mn(a_addr + kk * 2048) : smem_desc(a_addr + kk * 32);
+                const uint64_t db = MN ? smem_desc_mn(b_addr + kk * 2048) : smem_desc(b_addr + kk * 32);
                 const uint32_t accumulate = (step > 0 || kk > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -233,15 +251,13 @@ gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensor
             wait_parity(smem_u32(&full_bar[step % kRing]), uint32_t(step / kRing) & 1u);
     }
 
-    // The output layer's partial sums of each row (two halves of the columns), after the
-    // transpose tiles.
-    float* head_part = reinterpret_cast<float*>(base + 32 * 1024);
+    // The output layer's partial sums of each row (two halves of the columns).
+    float* head_part = reinterpret_cast<float*>(base);
     if (!aborted && steps > 0) {
         const int quarter = warp & 3, half = warp >> 2;
         const int m = row0 + quarter * 32 + lane;
         const bool valid = m < p.rows_a;
         float head = 0.f;
-        unsigned char* stage_t = base + warp * (32 * kTransposeStride);  // this warp's transpose tile
         for (int c0 = 32 * half; c0 < N; c0 += 64) {
             uint32_t r[32];
             const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(c0);
@@ -323,38 +339,27 @@ gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensor
                             head += h0.x * w.x + h0.y * w.y + h1.x * w.z + h1.y * w.w;
                         }
                     }
-                    if (p.HT) {
-                        // Transpose through shared memory: lane (row m) writes its 32 values down
-                        // a column of the warp's tile, then lane (column c0 + lane) writes the 32
-                        // rows of its column as 64 contiguous bytes.
-                        __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(stage_t);
+                    if (EPI == kBackward && p.bias_grad) {
+                        // Column sums of this warp's 32 rows (BF16-rounded, as stored): each
+                        // step halves the columns a lane holds and doubles the rows in them,
+                        // which leaves lane l with column c0 + l.
+                        float g[32];
 #pragma unroll
-                        for (int q = 0; q < 32; ++q)
-                            tile[q * (kTransposeStride / 2) + lane] = valid ? __float2bfloat16(v[q]) : __float2bfloat16(0.f);
-                        __syncwarp();
-                        const int m0 = row0 + quarter * 32;
-                        const uint4* row = reinterpret_cast<const uint4*>(stage_t + lane * kTransposeStride);
-                        __nv_bfloat16* dst = p.HT + size_t(c0 + lane) * p.rows_ht + m0;
-                        if (m0 + 32 <= p.rows_ht) {
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(dst)[q] = row[q];
-                        } else {
-                            const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(row);
-                            for (int q = 0; m0 + q < p.rows_ht; ++q) dst[q] = src[q];
+                        for (int q = 0; q < 16; ++q) {
+                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&packed[q]));
+                            g[2 * q] = valid ? f.x : 0.f;
+                            g[2 * q + 1] = valid ? f.y : 0.f;
                         }
-                        if (EPI == kBackward && p.bias_grad) {
-                            // Column c0 + lane of G over this warp's 32 rows (rows past rows_a
-                            // were staged as zeros).
-                            const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(row);
-                            float sum = 0.f;
 #pragma unroll
-                            for (int q = 0; q < 16; ++q) {
-                                const float2 f = __bfloat1622float2(g2[q]);
-                                sum += f.x + f.y;
+                        for (int off = 16; off > 0; off >>= 1) {
+                            const bool upper = lane & off;
+#pragma unroll
+                            for (int q = 0; q < off; ++q) {
+                                const float give = upper ? g[q] : g[q + off], keep = upper ? g[q + off] : g[q];
+                                g[q] = keep + __shfl_xor_sync(0xffffffffu, give, off);
                             }
-                            atomicAdd(p.bias_grad + c0 + lane, sum);
                         }
-                        __syncwarp();
+                        atomicAdd(p.bias_grad + c0 + lane, g[0]);
                     }
                 }
                 continue;
@@ -375,12 +380,10 @@ gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensor
                     p.Z[e] = __float2bfloat16(z);
                     const __nv_bfloat16 h = __float2bfloat16(gelu(z));
                     p.H[e] = h;
-                    if (p.HT) p.HT[size_t(n) * p.rows_ht + m] = h;
                     if (p.head_w) head += __bfloat162float(h) * p.head_w[n];
                 } else {
                     const __nv_bfloat16 g = __float2bfloat16(acc * gelu_grad(__bfloat162float(p.zprev[e])));
                     p.H[e] = g;
-                    if (p.HT) p.HT[size_t(n) * p.rows_ht + m] = g;
                     if (p.bias_grad) atomicAdd(p.bias_grad + n, __bfloat162float(g));
                 }
             }
