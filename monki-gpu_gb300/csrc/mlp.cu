@@ -192,6 +192,8 @@ struct Net {
     float* loss = nullptr;
     uint32_t* failure = nullptr;
     uint32_t* idx = nullptr;
+    // Device copies of a call's host rows (up to R), made at the first call that needs them.
+    float *in_x = nullptr, *in_t = nullptr, *in_w = nullptr;
     float *data_x = nullptr, *data_t = nullptr, *data_w = nullptr;
     uint32_t data_n = 0;
     uint32_t step = 0, seed = 0;
@@ -204,6 +206,13 @@ struct Net {
         check(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(P)), "cudaMalloc");
         owned.push_back(p);
         return static_cast<P*>(p);
+    }
+    void input_rows() {
+        if (!in_x) in_x = alloc<float>(size_t(R) * size_t(features));
+    }
+    void input_targets() {
+        if (!in_t) in_t = alloc<float>(size_t(R));
+        if (!in_w) in_w = alloc<float>(size_t(R));
     }
     ~Net() {
         if (stream) cudaStreamSynchronize(stream);
@@ -456,23 +465,16 @@ int monki_mlp_forward(void* handle, const float* x, uint32_t rows, float* y, cha
     try {
         if (!n || (!x && rows) || (!y && rows)) throw std::runtime_error("Invalid network or buffers");
         check(cudaSetDevice(n->device), "cudaSetDevice");
-        float* dx = nullptr;
-        check(cudaMalloc(&dx, std::max<size_t>(1, size_t(std::min<uint32_t>(rows, uint32_t(n->R))) * n->features * sizeof(float))), "cudaMalloc");
-        try {
-            for (uint32_t r0 = 0; r0 < rows; r0 += uint32_t(n->R)) {
-                const int m = int(std::min<uint32_t>(uint32_t(n->R), rows - r0));
-                check(cudaMemcpyAsync(dx, x + size_t(r0) * n->features, size_t(m) * n->features * sizeof(float),
-                                      cudaMemcpyHostToDevice, n->stream), "upload");
-                pack_rows(*n, dx, nullptr, m);
-                forward(*n, m);
-                check(cudaMemcpyAsync(y + r0, n->y, size_t(m) * sizeof(float), cudaMemcpyDeviceToHost, n->stream), "download");
-                check_failure(*n);
-            }
-        } catch (...) {
-            cudaFree(dx);
-            throw;
+        if (rows) n->input_rows();
+        for (uint32_t r0 = 0; r0 < rows; r0 += uint32_t(n->R)) {
+            const int m = int(std::min<uint32_t>(uint32_t(n->R), rows - r0));
+            check(cudaMemcpyAsync(n->in_x, x + size_t(r0) * n->features, size_t(m) * n->features * sizeof(float),
+                                  cudaMemcpyHostToDevice, n->stream), "upload");
+            pack_rows(*n, n->in_x, nullptr, m);
+            forward(*n, m);
+            check(cudaMemcpyAsync(y + r0, n->y, size_t(m) * sizeof(float), cudaMemcpyDeviceToHost, n->stream), "download");
+            check_failure(*n);
         }
-        cudaFree(dx);
         return 0;
     } catch (const std::exception& e) {
         write_error(err, errlen, e.what());
@@ -491,15 +493,13 @@ int monki_mlp_gradients(void* handle, const float* x, const float* target, const
         for (uint32_t m = 0; m < rows; ++m) total += weight[m];
         if (!(total > 0.0)) throw std::runtime_error("Weights must have a positive sum");
         check(cudaSetDevice(n->device), "cudaSetDevice");
-        float *dx = nullptr, *dt = nullptr, *dw = nullptr;
-        check(cudaMalloc(&dx, size_t(rows) * n->features * sizeof(float)), "cudaMalloc");
-        check(cudaMalloc(&dt, rows * sizeof(float)), "cudaMalloc");
-        check(cudaMalloc(&dw, rows * sizeof(float)), "cudaMalloc");
-        check(cudaMemcpyAsync(dx, x, size_t(rows) * n->features * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
-        check(cudaMemcpyAsync(dt, target, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
-        check(cudaMemcpyAsync(dw, weight, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
-        pack_rows(*n, dx, nullptr, int(rows));
-        gather_targets<<<256, 256, 0, n->stream>>>(dt, dw, nullptr, int(rows), n->R, n->tb, n->wb);
+        n->input_rows();
+        n->input_targets();
+        check(cudaMemcpyAsync(n->in_x, x, size_t(rows) * n->features * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
+        check(cudaMemcpyAsync(n->in_t, target, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
+        check(cudaMemcpyAsync(n->in_w, weight, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
+        pack_rows(*n, n->in_x, nullptr, int(rows));
+        gather_targets<<<256, 256, 0, n->stream>>>(n->in_t, n->in_w, nullptr, int(rows), n->R, n->tb, n->wb);
         check(cudaMemsetAsync(n->grads, 0, kParams * sizeof(float), n->stream), "memset");
         check(cudaMemsetAsync(n->loss, 0, sizeof(float), n->stream), "memset");
         forward(*n, int(rows));
@@ -507,7 +507,6 @@ int monki_mlp_gradients(void* handle, const float* x, const float* target, const
         check(cudaMemcpyAsync(grads, n->grads, kParams * sizeof(float), cudaMemcpyDeviceToHost, n->stream), "download");
         check(cudaMemcpyAsync(loss, n->loss, sizeof(float), cudaMemcpyDeviceToHost, n->stream), "download");
         check_failure(*n);
-        cudaFree(dx); cudaFree(dt); cudaFree(dw);
         return 0;
     } catch (const std::exception& e) {
         write_error(err, errlen, e.what());
