@@ -238,7 +238,8 @@ inline double analog_norm(const Prepared::Lut& l, int nmat) {
 }
 
 // Host image of the device scene: element offsets into one allocation of T, plus the
-// guide tables (int) appended after the T region.
+// guide tables (int) appended after the T region. Without `nodes` every species takes its
+// general tables (16 bytes per scattering angle less).
 template <typename T>
 struct Packed {
     std::vector<T> values;
@@ -251,7 +252,7 @@ struct Packed {
 };
 
 template <typename T>
-Packed<T> pack(const Prepared& p, bool uniform_prefix, bool rectangles = true) {
+Packed<T> pack(const Prepared& p, bool uniform_prefix, bool rectangles = true, bool nodes = true) {
     Packed<T> k{};
     auto& v = k.values;
     const size_t cols = size_t(p.nx) * p.ny, ncell = cols * p.nz;
@@ -391,7 +392,7 @@ Packed<T> pack(const Prepared& p, bool uniform_prefix, bool rectangles = true) {
         }
         // A species that does not polarize has one table: its nodes carry everything the
         // sampling and the phase function read, one vector load per node.
-        bool plain = true;
+        bool plain = nodes;
         for (int i = 0; i < l.n && plain; ++i) {
             const T f11 = T(l.f11[i]);
             plain = f11 >= T(0) && T(l.f22[i]) == f11 && T(l.f33[i]) == f11 && T(l.f12[i]) == T(0);

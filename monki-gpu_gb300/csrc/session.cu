@@ -1020,7 +1020,8 @@ extern "C" int monki_cuda_run_static(uint32_t device, const double* tables, size
 
         // Layout inside the array: packed scene, tally bank (one shard per round), FP64
         // output staging, mu0/mu per view, failure word and counters.
-        Packed<float> k = pack<float>(p, true);
+        // No node tables: scenes that fill the array leave no room for them.
+        Packed<float> k = pack<float>(p, true, true, false);
         TallyLayout L{};
         L.stokes = uint32_t(p.nmat * p.nx * p.ny * p.angles);
         L.paths = p.paths ? uint32_t(p.nx * p.ny * p.nz * p.angles) : 0u;
