@@ -192,8 +192,11 @@ struct Net {
     float* loss = nullptr;
     uint32_t* failure = nullptr;
     uint32_t* idx = nullptr;
-    // Device copies of a call's host rows (up to R), made at the first call that needs them.
-    float *in_x = nullptr, *in_t = nullptr, *in_w = nullptr;
+    // Device copies of a call's host rows, targets and weights: room for the most rows a call
+    // has had (at most R).
+    float* in_x = nullptr;
+    float *in_t = nullptr, *in_w = nullptr;
+    size_t in_rows = 0;
     float *data_x = nullptr, *data_t = nullptr, *data_w = nullptr;
     uint32_t data_n = 0;
     uint32_t step = 0, seed = 0;
@@ -207,17 +210,21 @@ struct Net {
         owned.push_back(p);
         return static_cast<P*>(p);
     }
-    void input_rows() {
-        if (!in_x) in_x = alloc<float>(size_t(R) * size_t(features));
-    }
-    void input_targets() {
-        if (!in_t) in_t = alloc<float>(size_t(R));
-        if (!in_w) in_w = alloc<float>(size_t(R));
+    void input_rows(size_t rows) {
+        if (rows <= in_rows) return;
+        check(cudaStreamSynchronize(stream), "sync");
+        cudaFree(in_x);
+        in_x = in_t = in_w = nullptr;
+        in_rows = 0;
+        check(cudaMalloc(&in_x, rows * size_t(features + 2) * sizeof(float)), "cudaMalloc");
+        in_t = in_x + rows * size_t(features);
+        in_w = in_t + rows;
+        in_rows = rows;
     }
     ~Net() {
         if (stream) cudaStreamSynchronize(stream);
         for (void* p : owned) cudaFree(p);
-        cudaFree(data_x); cudaFree(data_t); cudaFree(data_w);
+        cudaFree(data_x); cudaFree(data_t); cudaFree(data_w); cudaFree(in_x);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -465,7 +472,7 @@ int monki_mlp_forward(void* handle, const float* x, uint32_t rows, float* y, cha
     try {
         if (!n || (!x && rows) || (!y && rows)) throw std::runtime_error("Invalid network or buffers");
         check(cudaSetDevice(n->device), "cudaSetDevice");
-        if (rows) n->input_rows();
+        if (rows) n->input_rows(std::min<size_t>(rows, size_t(n->R)));
         for (uint32_t r0 = 0; r0 < rows; r0 += uint32_t(n->R)) {
             const int m = int(std::min<uint32_t>(uint32_t(n->R), rows - r0));
             check(cudaMemcpyAsync(n->in_x, x + size_t(r0) * n->features, size_t(m) * n->features * sizeof(float),
@@ -493,8 +500,7 @@ int monki_mlp_gradients(void* handle, const float* x, const float* target, const
         for (uint32_t m = 0; m < rows; ++m) total += weight[m];
         if (!(total > 0.0)) throw std::runtime_error("Weights must have a positive sum");
         check(cudaSetDevice(n->device), "cudaSetDevice");
-        n->input_rows();
-        n->input_targets();
+        n->input_rows(rows);
         check(cudaMemcpyAsync(n->in_x, x, size_t(rows) * n->features * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
         check(cudaMemcpyAsync(n->in_t, target, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
         check(cudaMemcpyAsync(n->in_w, weight, rows * sizeof(float), cudaMemcpyHostToDevice, n->stream), "upload");
