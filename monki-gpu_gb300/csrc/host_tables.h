@@ -238,8 +238,8 @@ inline double analog_norm(const Prepared::Lut& l, int nmat) {
 }
 
 // Host image of the device scene: element offsets into one allocation of T, plus the
-// guide tables (int) appended after the T region. Without `nodes` every species takes its
-// general tables (16 bytes per scattering angle less).
+// guide tables (int) appended after the T region. `nodes` adds the node tables of the plain
+// species (16 bytes per scattering angle) for the kernels that read them: the wavefront.
 template <typename T>
 struct Packed {
     std::vector<T> values;

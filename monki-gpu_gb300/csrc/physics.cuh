@@ -151,13 +151,17 @@ __device__ __forceinline__ T plain_f11(const T* __restrict__ node, int n, int lo
     return lut_lerp(cs, a.x, b.x, a.z, b.z) / T(4);
 }
 
-template <typename T>
+// NODES: a plain species reads its node table. The one-thread-per-history kernel takes the
+// general tables alone (NODES = false): both forms in its one loop cost it more than the node
+// table gives (box cloud with a polarizing cloud, 1.2 M photons 27.3 -> 35.4 ms with the branch,
+// with a plain one 26.5 -> 28.4), and its FP32 histories would round differently.
+template <typename T, bool NODES = true>
 __device__ __forceinline__ Phase<T> particle(const SceneView<T>& s, int sp, T cs, int nmat) {
     const int n = s.lut_n[sp];
     const T* __restrict__ cosv = s.lut_cos[sp];
     const T* __restrict__ f = s.lut_f[sp];
     const T* __restrict__ node = s.node[sp];
-    if (nmat < 4 && node) {
+    if (NODES && nmat < 4 && node) {
         // One lerp for the one table (its F22 and F33 lerps would repeat it, F12 stays 0).
         const T f11 = plain_f11<T>(node, n, lut_guess<T>(n, cs), cs);
         return Phase<T>{f11, f11, f11, T(0), T(0), T(0)};
@@ -193,9 +197,9 @@ __device__ __forceinline__ Phase<T> particle(const SceneView<T>& s, int sp, T cs
     return r;
 }
 
-template <typename T>
+template <typename T, bool NODES = true>
 __device__ __forceinline__ Phase<T> phase(const SceneView<T>& s, int sp, T cs, int nmat) {
-    return sp < 0 ? rayleigh<T>(cs, s.depol, nmat) : particle<T>(s, sp, cs, nmat);
+    return sp < 0 ? rayleigh<T>(cs, s.depol, nmat) : particle<T, NODES>(s, sp, cs, nmat);
 }
 
 // ---------------------------------------------------------------------------------
@@ -349,13 +353,13 @@ __device__ __forceinline__ T sample_cdf(const SceneView<T>& s, int sp, T u) {
 // box-cloud round (126.5 against 127.2 ms), but the Stokes update then rounds differently and
 // about one history in 10^9 scatters takes another path. The node records took the same round
 // (50,000 photons per column, 30 x 20 columns) from 145.1 to 129 ms.
-template <typename T, typename Stream>
+template <typename T, bool NODES = true, typename Stream>
 __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, int nmat, const T* st,
                                                  T cos_in, Stream& rng, T& cos_out, T& dphi,
                                                  T& cos_sca, T sign = T(-1)) {
     const T pi = pi_v<T>();
     float u[3];
-    if (sp >= 0 && nmat < 4 && s.node[sp]) {
+    if (NODES && sp >= 0 && nmat < 4 && s.node[sp]) {
         // A plain species: its proposal is its phase function, so the first draw is always
         // accepted (pdf and bound are both F11; the acceptance draw is spent all the same).
         const int n = s.lut_n[sp];
@@ -379,7 +383,7 @@ __device__ __forceinline__ bool sample_direction(const SceneView<T>& s, int sp, 
         T u1 = T(u[0]);
         T cs = sp < 0 ? T(2) * u1 - T(1) : sample_cdf<T>(s, sp, u1);
         T sigma = T(2) * pi * T(u[1]) - pi;
-        Phase<T> f = phase<T>(s, sp, cs, nmat);
+        Phase<T> f = phase<T, NODES>(s, sp, cs, nmat);
         T pdf = f.f11;
         if (nmat > 1) {
             T s2, c2;

@@ -81,7 +81,7 @@ struct Session {
 
 template <typename T>
 void upload(Session& s) {
-    Packed<T> k = pack<T>(s.prep, s.cfg.uniform_prefix, s.cfg.rectangles);
+    Packed<T> k = pack<T>(s.prep, s.cfg.uniform_prefix, s.cfg.rectangles, s.cfg.wavefront);
     size_t bytes = k.values.size() * sizeof(T) + k.guides.size() * sizeof(int);
     check(cudaMalloc(&s.scene, std::max<size_t>(bytes, 16)), "cudaMalloc(scene)");
     // Stream-ordered copies, complete before the host image goes out of scope.
@@ -1024,7 +1024,7 @@ extern "C" int monki_cuda_run_static(uint32_t device, const double* tables, size
 
         // Layout inside the array: packed scene, tally bank (one shard per round), FP64
         // output staging, mu0/mu per view, failure word and counters.
-        // No node tables: scenes that fill the array leave no room for them.
+        // No node tables: this kernel does not read them.
         Packed<float> k = pack<float>(p, true, true, false);
         TallyLayout L{};
         L.stokes = uint32_t(p.nmat * p.nx * p.ny * p.angles);

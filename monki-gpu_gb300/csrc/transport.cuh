@@ -235,7 +235,7 @@ transport_kernel(SceneView<T> s, Controls ctl, TA* __restrict__ banks, TallyLayo
                 T cs = c * vc + sqrt(fmax(eps, T(1) - c * c)) * sqrt(fmax(eps, T(1) - vc * vc)) *
                                     cos(phi - s.vphi[ia]);
                 Rot<T> r = NMAT > 1 ? rotation<T>(cs, c, vc, phi, s.vphi[ia]) : Rot<T>{T(1), T(0), T(1), T(0)};
-                Phase<T> f = phase<T>(s, sp, cs, NMAT);
+                Phase<T> f = phase<T, false>(s, sp, cs, NMAT);
                 T back[3];
                 scatter_stokes<T>(f, r, NMAT, st, back);
                 for (int m = 0; m < NMAT; ++m) prob[m] = back[m] * weight;
@@ -251,13 +251,13 @@ transport_kernel(SceneView<T> s, Controls ctl, TA* __restrict__ banks, TallyLayo
             }
             if (flag) break;
             T cos_out, dphi, cos_sca;
-            if (!sample_direction<T>(s, sp, NMAT, st, c, rng, cos_out, dphi, cos_sca)) {
+            if (!sample_direction<T, false>(s, sp, NMAT, st, c, rng, cos_out, dphi, cos_sca)) {
                 flag = kSamplingCap; break;
             }
             const T phi_out = phi + dphi;
             {
                 Rot<T> r = NMAT > 1 ? rotation<T>(cos_sca, c, cos_out, phi, phi_out) : Rot<T>{T(1), T(0), T(1), T(0)};
-                Phase<T> f = phase<T>(s, sp, cos_sca, NMAT);
+                Phase<T> f = phase<T, false>(s, sp, cos_sca, NMAT);
                 T ns[3];
                 scatter_stokes<T>(f, r, NMAT, st, ns);
                 const T s0 = ns[0];
