@@ -199,13 +199,17 @@ void upload_scene(Multi& m, Scene& sc, cudaStream_t stream) {
     if constexpr (sizeof(T) == 4) sc.view32 = v; else sc.view64 = v;
 }
 
+void drop_graph(Group& g) {
+    if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
+    if (g.graph) { cudaGraphDestroy(g.graph); g.graph = nullptr; }
+}
+
 void destroy(Multi* m) {
     if (!m) return;
     cudaSetDevice(m->device);
     for (Group& g : m->groups) {
         if (g.stream) cudaStreamSynchronize(g.stream);
-        if (g.exec) cudaGraphExecDestroy(g.exec);
-        if (g.graph) cudaGraphDestroy(g.graph);
+        drop_graph(g);
         cudaFree(g.pool); cudaFree(g.entries); cudaFree(g.block_scene);
         if (g.host_entries) cudaFreeHost(g.host_entries);
         if (g.host_block_scene) cudaFreeHost(g.host_block_scene);
@@ -281,8 +285,9 @@ void lay_out(Multi& m, Group& g, const std::vector<Controls>& ctl) {
 // Launch blocks for the entries that each scene's lists can still hold: all of its slots until
 // its photons are claimed, then the live ones (none is added). Between two batches of a group,
 // each time half of the blocks would be idle (16 scenes of 63.6 M photons: 769 -> 761 ms).
+// True when the launches changed, and with them the group's graph.
 template <typename T>
-void shrink(Group& g, const std::vector<Controls>& ctl) {
+bool shrink(Group& g, const std::vector<Controls>& ctl) {
     SceneEntry<T>* entries = static_cast<SceneEntry<T>*>(g.host_entries);
     auto needed = [&](size_t q) {
         const Controls& c = ctl[size_t(g.members[q])];
@@ -294,7 +299,7 @@ void shrink(Group& g, const std::vector<Controls>& ctl) {
     };
     uint32_t total = 0;
     for (size_t q = 0; q < g.members.size(); ++q) total += needed(q);
-    if (!total || total > g.blocks / 2) return;
+    if (!total || total > g.blocks / 2) return false;
     uint32_t block = 0;
     for (size_t q = 0; q < g.members.size(); ++q) {
         const uint32_t blocks = needed(q);
@@ -308,7 +313,7 @@ void shrink(Group& g, const std::vector<Controls>& ctl) {
                           g.stream), "upload(entries)");
     check(cudaMemcpyAsync(g.block_scene, g.host_block_scene, block * sizeof(uint16_t), cudaMemcpyHostToDevice, g.stream),
           "upload(blocks)");
-    if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }  // launches of this size from here on
+    return true;
 }
 
 // Graph (or stream launches) of one batch of check_every wavefront iterations of a group:
@@ -372,6 +377,18 @@ void batch(Multi& m, Group& g, cudaStream_t stream, cudaGraph_t graph) {
     }
 }
 
+// The group's batch at its present launch size as a graph. A shrunk batch is rebuilt, at most
+// once per halving: launched kernel by kernel it was slower than the full-size graph wherever
+// the drain is long (without tail launches, full-size graph / launches / rebuilt graph: 4 scenes
+// of 11.7 M scatters 131 / 154 / 125 ms, 8 of 45 M 106 / 108 / 88 ms).
+template <typename T>
+void build_graph(Multi& m, Group& g) {
+    drop_graph(g);
+    check(cudaGraphCreate(&g.graph, 0), "graph create");
+    if (g.nmat == 1) batch<T, 1>(m, g, g.stream, g.graph); else batch<T, 3>(m, g, g.stream, g.graph);
+    check(cudaGraphInstantiate(&g.exec, g.graph, 0), "graph instantiate");
+}
+
 template <typename T>
 void set_attributes(const Group& g) {
     // Shared memory: the staged band (dynamic) plus the entry and the kernels' own statics.
@@ -386,8 +403,7 @@ void set_attributes(const Group& g) {
 template <typename T>
 void run(Multi& m, const std::vector<Controls>& ctl) {
     for (Group& g : m.groups) {
-        if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
-        if (g.graph) { cudaGraphDestroy(g.graph); g.graph = nullptr; }
+        drop_graph(g);
         g.active = false;
         bool any = false;
         for (int id : g.members) any = any || ctl[size_t(id)].count > 0;
@@ -395,11 +411,7 @@ void run(Multi& m, const std::vector<Controls>& ctl) {
         lay_out<T>(m, g, ctl);
         wf_reset_multi<T><<<g.blocks, kMultiBlock, 0, g.stream>>>(static_cast<const SceneEntry<T>*>(g.entries), g.block_scene);
         check(cudaGetLastError(), "reset launch");
-        if (m.cfg.graphs) {
-            check(cudaGraphCreate(&g.graph, 0), "graph create");
-            if (g.nmat == 1) batch<T, 1>(m, g, g.stream, g.graph); else batch<T, 3>(m, g, g.stream, g.graph);
-            check(cudaGraphInstantiate(&g.exec, g.graph, 0), "graph instantiate");
-        }
+        if (m.cfg.graphs) build_graph<T>(m, g);
         g.active = true;
     }
     uint64_t it = 0, launches = 0;
@@ -454,7 +466,7 @@ void run(Multi& m, const std::vector<Controls>& ctl) {
                 done = true;
             }
             if (done) g.active = false;
-            else shrink<T>(g, ctl);
+            else if (shrink<T>(g, ctl) && m.cfg.graphs) build_graph<T>(m, g);
         }
         if (it > limit * 4 + 1024 && it > 1000000) throw std::runtime_error("multi-scene wavefront did not drain");
     }

@@ -1,0 +1,119 @@
+"""Host code of the multi-scene session (csrc/multi.cu, csrc/tail.cu) over a runtime of host
+memory: the order of its calls and what it does when one fails, with the read-back counts of
+each wavefront batch supplied by the test.
+"""
+
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+COUNT_WORDS, CLAIMED = 20, 16  # words per scene of the read-back counts; index of the claim counter
+LAUNCH_FAILED = 719
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    import fake_cuda
+
+    return fake_cuda.build(tmp_path_factory.mktemp("host"), ("multi", "tail"))
+
+
+class Session:
+    """A multi-scene session of one scene per group (I, and I/Q/U). ``live[group]`` lists the
+    photons left after each batch, every photon claimed from the second batch on; a group whose
+    list has ended has none left."""
+
+    def __init__(self, library, config, live=((), ())):
+        import fake_cuda
+        import monki.scenes as scenes
+
+        self.runtime = fake_cuda.Runtime(library)
+        self.native = self.runtime.library
+        self.native.monki_cuda_multi_create.restype = ctypes.c_void_p
+        self.native.monki_cuda_multi_tally_count.restype = ctypes.c_size_t
+        self.scenes = [scenes.clear_sky(2000, 1, nx=12, ny=10),
+                       scenes.box_cloud(2000, 1, nx=15, ny=11, box_x=(3, 8), box_y=(2, 6))]
+        self.photons = [s.photons_per_column * s.shape[1] * s.shape[2] for s in self.scenes]
+        tables = [np.ascontiguousarray(s.tables) for s in self.scenes]
+        f64p = ctypes.POINTER(ctypes.c_double)
+        pointers = (f64p * 2)(*[t.ctypes.data_as(f64p) for t in tables])
+        sizes = (ctypes.c_size_t * 2)(*[t.size for t in tables])
+        self.error = ctypes.create_string_buffer(2048)
+        self.handle = self.native.monki_cuda_multi_create(0, 2, pointers, sizes, 1, config.encode(), self.error, 2048)
+        assert self.handle, self.error.value
+        # The pinned count buffers: the groups' host_counts, in the order of their creation.
+        self.counts = [e.pointer for e in self.runtime.events if e.call == "malloc host" and e.value == 4 * COUNT_WORDS]
+        assert len(self.counts) == 2
+        self.batches = [0, 0]
+        self.live = live
+        self.fail = lambda event: 0
+        self.runtime.on_call = self._on_call
+
+    def _on_call(self, event):
+        if event.call == "copy" and event.pointer in self.counts:
+            group = self.counts.index(event.pointer)
+            words = (ctypes.c_uint32 * COUNT_WORDS).from_address(event.pointer)
+            batch, left = self.batches[group], self.live[group]
+            ctypes.memset(words, 0, ctypes.sizeof(words))
+            words[2] = left[batch] if batch < len(left) else 0
+            words[CLAIMED] = self.photons[group] if batch else 0
+            self.batches[group] = batch + 1
+        return self.fail(event)
+
+    def run(self):
+        controls = np.zeros((2, 8), dtype=np.uint32)
+        for q, photons in enumerate(self.photons):
+            controls[q] = [photons, 0, 1, 7, 100000, 0, photons, 1]
+        outs = [np.zeros(self.native.monki_cuda_multi_tally_count(ctypes.c_void_p(self.handle), q)) for q in range(2)]
+        f64p = ctypes.POINTER(ctypes.c_double)
+        out = (f64p * 2)(*[o.ctypes.data_as(f64p) for o in outs])
+        self.first = len(self.runtime.events)
+        return self.native.monki_cuda_multi_run(ctypes.c_void_p(self.handle), controls.ctypes.data_as(ctypes.c_void_p),
+                                                out, self.error, 2048)
+
+    def of_run(self):
+        return self.runtime.events[self.first :]
+
+    def close(self):
+        self.native.monki_cuda_multi_close(ctypes.c_void_p(self.handle))
+        self.runtime.close()
+
+
+def _grids(events, kernel):
+    grids = []
+    for e in events:
+        if kernel in e.kernel and (not grids or grids[-1] != e.grid):
+            grids.append(e.grid)
+    return grids
+
+
+def test_shrunk_launches_replay_a_graph(library):
+    """The launches of a group that is draining cover its live entries, and stay graph replays:
+    launched kernel by kernel, a drain without tail launches took longer than with full-size
+    graphs (four small scenes 131 ms with those, 154 launched one by one)."""
+
+    session = Session(library, "pool=262144,check_every=2,tail=0,graphs=1",
+                      live=((240000, 100000, 5000, 300), (330000, 330000, 200)))
+    assert session.run() == 0, session.error.value
+    wavefront = [e for e in session.of_run() if "wf_step_multi" in e.kernel or "wf_peel_multi" in e.kernel]
+    assert {e.call for e in wavefront} == {"graph kernel"}
+    streams = list(dict.fromkeys(e.stream for e in wavefront))
+    full = [-(-p // 256) for p in (240000, 262144)]
+    for kernel in ("wf_step_multi", "wf_peel_multi"):
+        first, second = ([e for e in wavefront if e.stream == s] for s in streams)
+        assert _grids(first, kernel) == [full[0], -(-100000 // 256), -(-5000 // 256), 2]
+        assert _grids(second, kernel) == [full[1], 1]
+    session.close()
+
+
+def test_without_graphs_shrunk_launches_are_launched_directly(library):
+    session = Session(library, "pool=262144,check_every=2,tail=0,graphs=0", live=((240000, 100000, 5000), (200, 0)))
+    assert session.run() == 0, session.error.value
+    assert not [e for e in session.of_run() if e.call.startswith("graph")]
+    step = [e for e in session.of_run() if "wf_step_multi" in e.kernel]
+    first = [e for e in step if e.stream == step[0].stream]
+    assert _grids(first, "wf_step_multi") == [-(-240000 // 256), -(-100000 // 256), -(-5000 // 256)]
+    session.close()
