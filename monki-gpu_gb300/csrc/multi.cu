@@ -204,11 +204,20 @@ void drop_graph(Group& g) {
     if (g.graph) { cudaGraphDestroy(g.graph); g.graph = nullptr; }
 }
 
+// Wait for whatever the session still has in flight: a run that fails leaves launches of other
+// groups and tails behind, which write the pool and the tally banks.
+void settle(const Multi& m) {
+    for (const Group& g : m.groups)
+        if (g.stream) cudaStreamSynchronize(g.stream);
+    for (cudaStream_t t : m.tail_streams)
+        if (t) cudaStreamSynchronize(t);
+}
+
 void destroy(Multi* m) {
     if (!m) return;
     cudaSetDevice(m->device);
+    settle(*m);
     for (Group& g : m->groups) {
-        if (g.stream) cudaStreamSynchronize(g.stream);
         drop_graph(g);
         cudaFree(g.pool); cudaFree(g.entries); cudaFree(g.block_scene);
         if (g.host_entries) cudaFreeHost(g.host_entries);
@@ -217,7 +226,8 @@ void destroy(Multi* m) {
         if (g.stream) cudaStreamDestroy(g.stream);
     }
     for (Scene& sc : m->scenes) { cudaFree(sc.tables); cudaFree(sc.banks); cudaFree(sc.out); cudaFree(sc.info); }
-    for (cudaStream_t t : m->tail_streams) { cudaStreamSynchronize(t); cudaStreamDestroy(t); }
+    for (cudaStream_t t : m->tail_streams)
+        if (t) cudaStreamDestroy(t);
     cudaFree(m->failure); cudaFree(m->counters); cudaFree(m->tail_next);
     if (m->t0) cudaEventDestroy(m->t0);
     if (m->t1) cudaEventDestroy(m->t1);
@@ -661,6 +671,7 @@ int monki_cuda_multi_run(void* handle, const uint32_t* controls, double* const* 
         m->totals[5] += m->scenes.size();  // the flushes
         return 0;
     } catch (const std::exception& e) {
+        settle(*m);
         write_error(err, errlen, e.what());
         return 1;
     }

@@ -117,3 +117,43 @@ def test_without_graphs_shrunk_launches_are_launched_directly(library):
     first = [e for e in step if e.stream == step[0].stream]
     assert _grids(first, "wf_step_multi") == [-(-240000 // 256), -(-100000 // 256), -(-5000 // 256)]
     session.close()
+
+
+@pytest.mark.parametrize("graphs", [1, 0])
+@pytest.mark.parametrize("failing", ["launch", "shrink"])
+def test_a_failed_run_waits_for_the_tails_it_launched(library, graphs, failing):
+    """The first group's tail is launched, then a call of the second group fails: the run ends
+    only after the tail, which writes the pool and the tally banks that the next run resets."""
+
+    session = Session(library, f"pool=262144,check_every=2,tail=65536,graphs={graphs}",
+                      live=((240000, 100), (330000, 300000, 100000, 80000)))
+
+    def fail(event):
+        events = session.of_run()
+        if not any("wf_tail" in e.kernel for e in events):
+            return 0
+        if failing == "launch":
+            return LAUNCH_FAILED if "wf_step_multi" in event.kernel or event.call == "graph launch" else 0
+        return LAUNCH_FAILED if event.call == "copy" and event.pointer not in session.counts else 0
+
+    session.fail = fail
+    assert session.run() == 1
+    assert b"failed by the test" in session.error.value
+    events = session.of_run()
+    tails = [n for n, e in enumerate(events) if "wf_tail" in e.kernel]
+    assert tails
+    for n in tails:
+        assert any(e.call == "synchronize" and e.stream == events[n].stream for e in events[n:])
+    session.close()
+
+
+def test_close_waits_for_every_stream_before_it_frees(library):
+    session = Session(library, "pool=262144,check_every=2", live=((240000, 100), (330000, 200)))
+    streams = {e.stream for e in session.runtime.events if e.call == "stream"}
+    assert session.run() == 0, session.error.value
+    first = len(session.runtime.events)
+    session.native.monki_cuda_multi_close(ctypes.c_void_p(session.handle))
+    events = session.runtime.events[first:]
+    freed = next(n for n, e in enumerate(events) if e.call.startswith("free"))
+    assert {e.stream for e in events[:freed] if e.call == "synchronize"} == streams
+    session.runtime.close()
