@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "host_tables.h"
+#include "launch.h"
 #include "tail.h"
 #include "wavefront.cuh"
 
@@ -406,8 +407,7 @@ void set_attributes(const Group& g) {
                                    : reinterpret_cast<const void*>(&wf_step_multi<T, 3>);
     const void* peel = g.nmat == 1 ? reinterpret_cast<const void*>(&wf_peel_multi<T, 1>)
                                    : reinterpret_cast<const void*>(&wf_peel_multi<T, 3>);
-    for (const void* fn : {step, peel})
-        check(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBandMaxBytes)), "attribute");
+    for (const void* fn : {step, peel}) check(allow_band(fn), "attribute");
 }
 
 template <typename T>

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 
+#include "launch.h"
 #include "tail.h"
 #include "wavefront.cuh"
 
@@ -21,8 +22,7 @@ cudaError_t launch(const SceneView<T>& v, const Controls& c, const Divisors& dv,
     int device = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess && v.band_bytes)
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(v.band_bytes));
+    if (e == cudaSuccess && v.band_bytes) e = allow_band(fn);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTailBlock, v.band_bytes);
     if (e != cudaSuccess) return e;
     // One resident wave: the blocks take slots until none is left.

@@ -157,3 +157,15 @@ def test_close_waits_for_every_stream_before_it_frees(library):
     freed = next(n for n, e in enumerate(events) if e.call.startswith("free"))
     assert {e.stream for e in events[:freed] if e.call == "synchronize"} == streams
     session.runtime.close()
+
+
+def test_a_tail_launch_lowers_no_other_sessions_shared_memory_limit(library):
+    """A kernel's dynamic shared-memory limit belongs to the kernel: sessions of other scenes
+    launch it from other threads, so no launch may set it to its own scene's band."""
+
+    session = Session(library, "pool=262144,check_every=2", live=((240000, 100), (330000, 200)))
+    assert session.run() == 0, session.error.value
+    tails = [e for e in session.of_run() if "wf_tail" in e.kernel and e.call == "launch"]
+    assert any(e.value > 0 for e in tails)  # a staged band
+    assert {e.value for e in session.runtime.events if e.call == "attribute"} <= {48 * 1024}
+    session.close()
