@@ -195,6 +195,11 @@ int monki_cuda_probe_scatter_stokes(uint32_t device, int fp64, double depol,
                                     const double *geometry, const double *stokes, uint32_t n,
                                     double *out, char *err, size_t errlen);
 
+/* The failure flags of a round group's first step launch on `blocks` blocks (FP32 forward I/Q/U
+ * scenes without layer paths): a launch too small for its work lists must be reported. */
+int monki_cuda_probe_step(void *session, const uint32_t controls[8], uint32_t blocks, uint32_t *failure, char *err,
+                          size_t errlen);
+
 #ifdef __cplusplus
 }
 #endif

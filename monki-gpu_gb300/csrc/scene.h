@@ -47,7 +47,7 @@ enum Failure : uint32_t {
     kSamplingCap = 4u,
     kInvalidStokes = 8u,
     kHistoryCap = 16u,
-    kQueueCorrupt = 32u,  // a queue entry outside the photon pool (internal error)
+    kQueueCorrupt = 32u,  // a queue entry outside the photon pool, or more than a launch serves (internal error)
     kStageTimeout = 64u,  // the shared-memory staging copy did not complete in time
 };
 

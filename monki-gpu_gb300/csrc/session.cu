@@ -897,6 +897,35 @@ int monki_cuda_importance(void* handle, double* out, size_t count, int reset, ch
     }
 }
 
+// Test hook: the first step launch of a round group on `blocks` blocks, its failure flags.
+int monki_cuda_probe_step(void* handle, const uint32_t controls[8], uint32_t blocks, uint32_t* failure, char* err,
+                          size_t errlen) {
+    Session* s = static_cast<Session*>(handle);
+    try {
+        if (!s || !controls || !failure || !blocks) throw std::runtime_error("Invalid CUDA session or probe");
+        if (!s->cfg.wavefront || s->cfg.fp64 || s->prep.paths || s->prep.backward || s->prep.nmat != 3)
+            throw std::runtime_error("the step probe runs FP32 forward I/Q/U scenes without layer paths");
+        const Controls c = group_controls(*s, controls);
+        check(cudaSetDevice(s->device), "cudaSetDevice");
+        Pool<float> P = s->pool32;
+        P.capacity = uint32_t(std::min<uint64_t>(P.capacity, (uint64_t(c.count) + 255) / 256 * 256));
+        const Divisors dv{FastDiv::make(c.per_round), FastDiv::make(uint32_t(s->prep.nx)),
+                          FastDiv::make(uint32_t(s->prep.ny)), FastDiv::make(uint32_t(s->prep.nx * s->prep.ny))};
+        check(cudaMemsetAsync(s->failure, 0, sizeof(uint32_t), s->stream), "memset(failure)");
+        wf_reset<float><<<int((P.capacity + 255) / 256), 256, 0, s->stream>>>(P);
+        check(cudaGetLastError(), "reset launch");
+        const Guide<float> g{0.f, 0.f, INFINITY, nullptr, 0.f};
+        Recorder{s->stream}.kernel(&wf_step<float, 3, false, false>, blocks, unsigned(s->cfg.block), s->view32.band_bytes,
+                                   s->view32, c, dv, P, g, s->cfg.walk, 0u, s->failure, s->counters);
+        check(cudaMemcpyAsync(failure, s->failure, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream), "copy(failure)");
+        check(cudaStreamSynchronize(s->stream), "step");
+        return 0;
+    } catch (const std::exception& e) {
+        write_error(err, errlen, e.what());
+        return 1;
+    }
+}
+
 int monki_cuda_inspect(const double* tables, size_t table_count, int fp64, int32_t* uniform_top,
                        double* tau_above, size_t tau_capacity, char* err, size_t errlen) {
     try {

@@ -1416,6 +1416,8 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
     // 37.6 -> 36.6 ms); with splitting a vacant slot may take a waiting copy instead.
     const uint32_t walks = events + held, entry0 = block * blockDim.x;
     if (threadIdx.x == 0) {
+        // One entry per thread below: a launch too small for its lists is refused.
+        if (total > blocks * blockDim.x) atomicOr(failure, kQueueCorrupt);
         claims_open = *reinterpret_cast<volatile uint32_t*>(P.counts + kClaimCount) < ctl.count;
         const uint32_t lo = max(entry0, walks), hi = min(entry0 + blockDim.x, total);
         first_claim = claims_open && !P.waiting && hi > lo ? atomicAdd(P.counts + kClaimCount, hi - lo) - lo : kNone;
@@ -1433,9 +1435,11 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
     __shared__ __align__(32) unsigned char hand[SCATTER && SMEM_HANDOFF ? 256 * kHandStride : 16];
     SlotState<T> local_state;
     SlotState<T>& state = SMEM_HANDOFF ? *reinterpret_cast<SlotState<T>*>(hand + threadIdx.x * kHandStride) : local_state;
-    // One entry per thread: the lists hold at most one per slot, and the launch covers the pool.
-    // The loop stays all the same: outside of one the compiler contracts the walk's arithmetic
-    // differently, which rounds differently and sends histories another way.
+    // One entry per thread: the lists hold at most one per slot, and the launch covers the pool or
+    // (multi-scene sessions, every photon claimed) the entries read back since, whose number only
+    // falls; a larger list was reported above. The loop stays all the same: outside of one the
+    // compiler contracts the walk's arithmetic differently, which rounds differently and sends
+    // histories another way.
     uint32_t slot = kNone;
     int list = -1;
     for (uint32_t e = block * blockDim.x + threadIdx.x; e < total; e += blocks * blockDim.x) {

@@ -119,6 +119,10 @@ _SIGNATURES = {
         ctypes.c_int,
         [ctypes.c_uint32, ctypes.c_int, ctypes.c_double, _F64P, _F64P, ctypes.c_uint32, _F64P, ctypes.c_char_p, ctypes.c_size_t],
     ),
+    "monki_cuda_probe_step": (
+        ctypes.c_int,
+        [ctypes.c_void_p, _U32P, ctypes.c_uint32, _U32P, ctypes.c_char_p, ctypes.c_size_t],
+    ),
 }
 
 EXPORTS = tuple(_SIGNATURES)
