@@ -52,8 +52,14 @@ void monki_mlp_close(void *net);
 
 /* Test hook: C (M x N, FP32) = A (M x K) B^T (N x K) from BF16 bit patterns through the
  * tcgen05 GEMM; K a multiple of 64, N a multiple of 16 in [16, 256]; splits > 1 splits K
- * (K / 64 divisible by splits) and accumulates. */
+ * (K / 64 divisible by splits) through the weight-gradient kernel. */
 int monki_mlp_gemm_probe(uint32_t device, const uint16_t *a, const uint16_t *b, int m, int n, int k, int splits,
+                         float *c, char *err, size_t errlen);
+
+/* Test hook of the weight-gradient kernel: C (M x N, FP32) = A^T B over the rows of A (rows x M)
+ * and B (rows x N), BF16 bit patterns, accumulated from slices of chunk rows (a multiple of
+ * 64); M a multiple of 128, N of 64 up to 256. */
+int monki_mlp_rows_probe(uint32_t device, const uint16_t *a, const uint16_t *b, int rows, int m, int n, int chunk,
                          float *c, char *err, size_t errlen);
 
 #ifdef __cplusplus

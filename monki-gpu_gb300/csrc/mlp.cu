@@ -235,12 +235,10 @@ bool g_attr_done[64] = {};
 void configure(int device) {
     std::lock_guard<std::mutex> guard(g_attr_lock);
     if (device < 0 || device >= 64 || g_attr_done[device]) return;
-    check(cudaFuncSetAttribute(umma::gemm<umma::kStore, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kForward, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kBackward, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kAccumulate, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               umma::smem_bytes_of<umma::kAccumulate>()), "attr");
-    check(cudaFuncSetAttribute(umma::gemm<umma::kAccumulate, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    check(cudaFuncSetAttribute(umma::gemm<umma::kStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kBackward>, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes), "attr");
+    check(cudaFuncSetAttribute(umma::gemm<umma::kAccumulate>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                umma::smem_bytes_of<umma::kAccumulate>()), "attr");
     g_attr_done[device] = true;
 }
@@ -294,8 +292,9 @@ struct Gemm {
 };
 
 // `rows` (MN-major): the valid rows; the tensor maps return zeros for those up to K.
-template <int EPI, bool MN = false>
+template <int EPI>
 void gemm(const Gemm& g, int splits, cudaStream_t stream, int rows = 0) {
+    constexpr bool MN = umma::mn_major<EPI>();
     const umma::Params& p = g.p;
     if (p.K % umma::kBlockK || p.k_chunk % umma::kBlockK || p.N % 16 || p.N < 16 || p.N > 256 || p.rows_a < 1 ||
         (MN && (p.N % 64 || p.rows_a % umma::kBlockM || rows < 1)))
@@ -305,7 +304,7 @@ void gemm(const Gemm& g, int splits, cudaStream_t stream, int rows = 0) {
     const CUtensorMap map_b = MN ? tile_map(g.B, rows, p.N, g.ldb, umma::kBlockK)
                                  : tile_map(g.B, p.N, p.K, g.ldb, p.N);
     dim3 grid((p.rows_a + umma::kBlockM - 1) / umma::kBlockM, splits);
-    umma::gemm<EPI, MN><<<grid, umma::kThreads, umma::smem_bytes_of<EPI>(), stream>>>(map_a, map_b, p);
+    umma::gemm<EPI><<<grid, umma::kThreads, umma::smem_bytes_of<EPI>(), stream>>>(map_a, map_b, p);
     check(cudaGetLastError(), "gemm launch");
 }
 
@@ -314,6 +313,16 @@ Gemm params_for(const bf16* A, const bf16* B, int rows, int N, int K, uint32_t* 
     g.p.rows_a = rows; g.p.N = N; g.p.K = K; g.p.k_chunk = K;
     g.p.failure = failure;
     return g;
+}
+
+// C (M x N) += A^T B over the rows of A (rows x M) and B (rows x N), split into slices of
+// `chunk` rows (a multiple of 64). M a multiple of 128, N of 64.
+void contract_rows(const bf16* A, const bf16* B, int rows, int M, int N, int chunk, float* C, uint32_t* failure,
+                   cudaStream_t stream) {
+    const int K = (rows + umma::kBlockK - 1) / umma::kBlockK * umma::kBlockK;
+    Gemm g = params_for(A, B, M, N, K, failure);
+    g.lda = M; g.ldb = N; g.p.k_chunk = chunk; g.p.C = C;
+    gemm<umma::kAccumulate>(g, (K + chunk - 1) / chunk, stream, rows);
 }
 
 void pack_rows(Net& n, const float* x, const uint32_t* idx, int rows) {
@@ -342,13 +351,10 @@ void backward(Net& n, int rows, float inv_weight, float* loss) {
     loss_grad<<<256, 256, 0, n.stream>>>(n.y, n.tb, n.wb, rows, inv_weight, n.dy, loss);
     head_backward<<<(rows + kSlab - 1) / kSlab, kHidden, 0, n.stream>>>(n.dy, n.H3, n.params + ow4, n.Z3, rows, n.grads, n.G3);
     check(cudaGetLastError(), "head backward launch");
-    // Split-K over the rows for the weight gradients: 64-row multiples, slices of 1,024 rows
-    // (at batch 65,536 two row tiles x 64 slices = 128 CTAs, each adding one partial).
-    const int chunk = 1024, K = (rows + 63) / 64 * 64, splits = (K + chunk - 1) / chunk;
+    // Slices of 1,024 rows for the weight gradients: at batch 65,536 two row tiles x 64 slices =
+    // 128 CTAs, each adding one partial.
     auto weight_gradient = [&](const bf16* dZ, const bf16* in, int width, float* out) {
-        Gemm g = params_for(dZ, in, kHidden, width, K, n.failure);
-        g.lda = kHidden; g.ldb = width; g.p.k_chunk = chunk; g.p.C = out;
-        gemm<umma::kAccumulate, true>(g, splits, n.stream, rows);
+        contract_rows(dZ, in, rows, kHidden, width, 1024, out, n.failure, n.stream);
     };
     auto input_gradient = [&](const bf16* dZ, const bf16* WT, const bf16* zprev, bf16* out, float* bias_grad) {
         Gemm g = params_for(dZ, WT, rows, kHidden, kHidden, n.failure);
@@ -373,6 +379,23 @@ void check_failure(Net& n) {
     check(cudaMemcpyAsync(&flag, n.failure, sizeof(flag), cudaMemcpyDeviceToHost, n.stream), "copy(failure)");
     check(cudaStreamSynchronize(n.stream), "mlp");
     if (flag) throw std::runtime_error("tensor-core GEMM wait gave up (flag " + std::to_string(flag) + ")");
+}
+
+// Device memory of a probe.
+template <typename P>
+struct Device {
+    P* p = nullptr;
+    explicit Device(size_t count) { check(cudaMalloc(&p, count * sizeof(P)), "cudaMalloc"); }
+    Device(const Device&) = delete;
+    Device& operator=(const Device&) = delete;
+    ~Device() { cudaFree(p); }
+};
+
+void read_probe(const Device<float>& from, const Device<uint32_t>& flag, size_t count, float* c) {
+    uint32_t f = 0;
+    check(cudaMemcpy(&f, flag.p, sizeof(f), cudaMemcpyDeviceToHost), "download");
+    check(cudaMemcpy(c, from.p, count * sizeof(float), cudaMemcpyDeviceToHost), "download");
+    if (f) throw std::runtime_error("tensor-core GEMM wait gave up");
 }
 
 }  // namespace mlp
@@ -596,36 +619,67 @@ void monki_mlp_close(void* handle) {
     delete n;
 }
 
-// Test hook: C (M x N, FP32) = A (M x K) B^T (N x K), BF16 bits in, through the tcgen05
-// GEMM; splits > 1 runs split-K into a zeroed C with the accumulating epilogue.
+// Test hook: C (M x N, FP32) = A^T B over the rows of A (rows x M) and B (rows x N), BF16 bits in,
+// through the weight-gradient kernel in slices of `chunk` rows. The rows up to the last tile's end
+// hold NaN on the device: no row past the valid ones may count.
+int monki_mlp_rows_probe(uint32_t device, const uint16_t* a, const uint16_t* b, int rows, int M, int N, int chunk,
+                         float* c, char* err, size_t errlen) {
+    try {
+        if (!a || !b || !c || rows < 1 || M < 128 || M % 128 || N < 64 || N % 64 || N > 256 || chunk < 64 || chunk % 64)
+            throw std::runtime_error("Invalid row contraction shape");
+        check(cudaSetDevice(int(device)), "cudaSetDevice");
+        configure(int(device));
+        const size_t held = (size_t(rows) + 63) / 64 * 64;
+        Device<bf16> da(held * M), db(held * N);
+        Device<float> dc(size_t(M) * N);
+        Device<uint32_t> flag(1);
+        check(cudaMemset(da.p, 0xFF, held * M * 2), "memset");
+        check(cudaMemset(db.p, 0xFF, held * N * 2), "memset");
+        check(cudaMemcpy(da.p, a, size_t(rows) * M * 2, cudaMemcpyHostToDevice), "upload");
+        check(cudaMemcpy(db.p, b, size_t(rows) * N * 2, cudaMemcpyHostToDevice), "upload");
+        check(cudaMemset(dc.p, 0, size_t(M) * N * 4), "memset");
+        check(cudaMemset(flag.p, 0, 4), "memset");
+        contract_rows(da.p, db.p, rows, M, N, chunk, dc.p, flag.p, nullptr);
+        read_probe(dc, flag, size_t(M) * N, c);
+        return 0;
+    } catch (const std::exception& e) {
+        write_error(err, errlen, e.what());
+        return 1;
+    }
+}
+
+// Test hook: C (M x N, FP32) = A (M x K) B^T (N x K), BF16 bits in, through the tcgen05 GEMM;
+// splits > 1 runs the weight-gradient kernel on the transposes, padded to its tiles.
 int monki_mlp_gemm_probe(uint32_t device, const uint16_t* a, const uint16_t* b, int M, int N, int K, int splits,
                          float* c, char* err, size_t errlen) {
     try {
         if (!a || !b || !c || M < 1 || splits < 1 || K % 64 || N % 16 || N < 16 || N > 256 || (K / 64) % splits)
             throw std::runtime_error("Invalid GEMM probe shape");
+        if (splits > 1) {
+            const int m = (M + 127) / 128 * 128, n = (N + 63) / 64 * 64;
+            std::vector<uint16_t> at(size_t(K) * m, 0), bt(size_t(K) * n, 0);
+            for (int k = 0; k < K; ++k) {
+                for (int r = 0; r < M; ++r) at[size_t(k) * m + r] = a[size_t(r) * K + k];
+                for (int r = 0; r < N; ++r) bt[size_t(k) * n + r] = b[size_t(r) * K + k];
+            }
+            std::vector<float> padded(size_t(m) * n);
+            if (monki_mlp_rows_probe(device, at.data(), bt.data(), K, m, n, K / splits, padded.data(), err, errlen)) return 1;
+            for (int r = 0; r < M; ++r) std::copy_n(padded.begin() + size_t(r) * n, N, c + size_t(r) * N);
+            return 0;
+        }
         check(cudaSetDevice(int(device)), "cudaSetDevice");
         configure(int(device));
-        bf16 *da = nullptr, *db = nullptr;
-        float* dc = nullptr;
-        uint32_t* flag = nullptr;
-        check(cudaMalloc(&da, size_t(M) * K * 2), "cudaMalloc");
-        check(cudaMalloc(&db, size_t(N) * K * 2), "cudaMalloc");
-        check(cudaMalloc(&dc, size_t(M) * N * 4), "cudaMalloc");
-        check(cudaMalloc(&flag, 4), "cudaMalloc");
-        check(cudaMemcpy(da, a, size_t(M) * K * 2, cudaMemcpyHostToDevice), "upload");
-        check(cudaMemcpy(db, b, size_t(N) * K * 2, cudaMemcpyHostToDevice), "upload");
-        check(cudaMemset(dc, 0, size_t(M) * N * 4), "memset");
-        check(cudaMemset(flag, 0, 4), "memset");
-        Gemm g = params_for(da, db, M, N, K, flag);
-        g.p.C = dc;
-        g.p.k_chunk = K / splits;
-        if (splits == 1) gemm<umma::kStore>(g, 1, nullptr);
-        else gemm<umma::kAccumulate>(g, splits, nullptr);
-        uint32_t f = 0;
-        check(cudaMemcpy(&f, flag, 4, cudaMemcpyDeviceToHost), "download");
-        check(cudaMemcpy(c, dc, size_t(M) * N * 4, cudaMemcpyDeviceToHost), "download");
-        cudaFree(da); cudaFree(db); cudaFree(dc); cudaFree(flag);
-        if (f) throw std::runtime_error("tensor-core GEMM wait gave up");
+        Device<bf16> da(size_t(M) * K), db(size_t(N) * K);
+        Device<float> dc(size_t(M) * N);
+        Device<uint32_t> flag(1);
+        check(cudaMemcpy(da.p, a, size_t(M) * K * 2, cudaMemcpyHostToDevice), "upload");
+        check(cudaMemcpy(db.p, b, size_t(N) * K * 2, cudaMemcpyHostToDevice), "upload");
+        check(cudaMemset(dc.p, 0, size_t(M) * N * 4), "memset");
+        check(cudaMemset(flag.p, 0, 4), "memset");
+        Gemm g = params_for(da.p, db.p, M, N, K, flag.p);
+        g.p.C = dc.p;
+        gemm<umma::kStore>(g, 1, nullptr);
+        read_probe(dc, flag, size_t(M) * N, c);
         return 0;
     } catch (const std::exception& e) {
         write_error(err, errlen, e.what());

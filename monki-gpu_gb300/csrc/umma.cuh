@@ -56,6 +56,10 @@ enum Epilogue : int {
 // The split-K weight-gradient GEMM runs one CTA per SM (its grid is about one wave) over 16
 // K steps, so it keeps four stages in flight instead of two.
 constexpr int kAccumulateStages = 4;
+// The weight gradients contract over the rows of both operands (MN-major), the others over the
+// columns (K-major).
+template <int EPI>
+constexpr bool mn_major() { return EPI == kAccumulate; }
 template <int EPI>
 constexpr int stages_of() { return EPI == kAccumulate ? kAccumulateStages : kStages; }
 template <int EPI>
@@ -163,11 +167,12 @@ __device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, i
 // Two CTAs per SM (128 registers): the unrolled GELU' of the backward epilogue takes 254 without
 // the bound, and one CTA per SM leaves nothing to run while it waits (backward GEMM of 65,536
 // rows 59.6 -> 47.4 us, 300 training steps 112.6 -> 104.7 ms).
-template <int EPI, bool MN>
+template <int EPI>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, Params p) {
     extern __shared__ __align__(1024) unsigned char raw[];
     constexpr int kRing = stages_of<EPI>();
+    constexpr bool MN = mn_major<EPI>();
     __shared__ __align__(8) uint64_t full_bar[kRing], empty_bar[kRing], done_bar;
     __shared__ uint32_t tmem_base;
     __shared__ int aborted;

@@ -89,6 +89,11 @@ _SIGNATURES = {
         [ctypes.c_uint32, ctypes.POINTER(ctypes.c_uint16), ctypes.POINTER(ctypes.c_uint16), ctypes.c_int, ctypes.c_int,
          ctypes.c_int, ctypes.c_int, _F32P, ctypes.c_char_p, ctypes.c_size_t],
     ),
+    "monki_mlp_rows_probe": (
+        ctypes.c_int,
+        [ctypes.c_uint32, ctypes.POINTER(ctypes.c_uint16), ctypes.POINTER(ctypes.c_uint16), ctypes.c_int, ctypes.c_int,
+         ctypes.c_int, ctypes.c_int, _F32P, ctypes.c_char_p, ctypes.c_size_t],
+    ),
     "monki_cuda_run_static": (
         ctypes.c_int,
         [ctypes.c_uint32, _F64P, ctypes.c_size_t, _U32P, _F64P, ctypes.c_char_p, ctypes.c_size_t],
