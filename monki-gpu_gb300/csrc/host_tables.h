@@ -42,6 +42,7 @@ struct Config {
     bool graphs = true;          // replay each batch of wavefront iterations as a CUDA graph
     bool orders = false;         // scattering-order diagnostics (single scattering, locations)
     bool rectangles = true;      // cross equal-extinction rectangles of the band in one step
+    bool nodes = true;           // node tables of plain species (0: their general tables, the same physics)
     uint32_t tail = 1u << 16;    // run a group's last photons to their end in one launch below this many (0 = off)
     int fused = -1;              // 1: scatter and walk in one step kernel; 0: separate kernels; -1: by scene
 };
@@ -101,6 +102,7 @@ inline Config parse_config(const char* text) {
         else if (key == "graphs") c.graphs = as_int(0, 1) != 0;
         else if (key == "orders") c.orders = as_int(0, 1) != 0;
         else if (key == "rectangles") c.rectangles = as_int(0, 1) != 0;
+        else if (key == "nodes") c.nodes = as_int(0, 1) != 0;
         else if (key == "tail") c.tail = uint32_t(as_int(0, 1l << 26));
         else if (key == "fused") c.fused = int(as_int(-1, 1));
         else throw std::runtime_error("Unknown config key: " + key);
@@ -239,7 +241,8 @@ inline double analog_norm(const Prepared::Lut& l, int nmat) {
 
 // Host image of the device scene: element offsets into one allocation of T, plus the
 // guide tables (int) appended after the T region. `nodes` adds the node tables of the plain
-// species (16 bytes per scattering angle) for the kernels that read them: the wavefront.
+// species (16 bytes per scattering angle) for the kernels that read them: the wavefront, up to
+// I/Q/U.
 template <typename T>
 struct Packed {
     std::vector<T> values;
@@ -392,7 +395,7 @@ Packed<T> pack(const Prepared& p, bool uniform_prefix, bool rectangles = true, b
         }
         // A species that does not polarize has one table: its nodes carry everything the
         // sampling and the phase function read, one vector load per node.
-        bool plain = nodes;
+        bool plain = nodes && p.nmat < 4;
         for (int i = 0; i < l.n && plain; ++i) {
             const T f11 = T(l.f11[i]);
             plain = f11 >= T(0) && T(l.f22[i]) == f11 && T(l.f33[i]) == f11 && T(l.f12[i]) == T(0);

@@ -187,7 +187,7 @@ size_t pool_bytes(size_t slots, size_t members, size_t record) {
 
 template <typename T>
 void upload_scene(Multi& m, Scene& sc, cudaStream_t stream) {
-    Packed<T> k = pack<T>(sc.prep, m.cfg.uniform_prefix, m.cfg.rectangles);
+    Packed<T> k = pack<T>(sc.prep, m.cfg.uniform_prefix, m.cfg.rectangles, m.cfg.nodes);
     const size_t bytes = k.values.size() * sizeof(T) + k.guides.size() * sizeof(int);
     check(cudaMalloc(&sc.tables, std::max<size_t>(bytes, 16)), "cudaMalloc(scene)");
     check(cudaMemcpyAsync(sc.tables, k.values.data(), k.values.size() * sizeof(T), cudaMemcpyHostToDevice, stream),

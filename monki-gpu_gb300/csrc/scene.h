@@ -18,7 +18,8 @@
 //   lut_cos[n], lut_cdf[n]   ascending cosine grid and the bound-function CDF
 //   lut_v[2 * n]             {F34, F44} per scattering angle, per species (nmat 4 only)
 //   node[4 * n]              {cosine, CDF, F11, 0} per scattering angle, for plain species
-//                            (F22 = F33 = F11 >= 0 and F12 = 0 at every angle); wavefront sessions
+//                            (F22 = F33 = F11 >= 0 and F12 = 0 at every angle) of wavefront
+//                            sessions up to I/Q/U
 //   guide[kGuide + 1]        CDF guide table: largest i with cdf[i] <= g / kGuide
 //   band[nx * ny * uniform_top]  extinction of every cell below the horizontally uniform
 //                            top (the only cells a cell walk visits), 16-byte aligned and

@@ -82,7 +82,7 @@ struct Session {
 
 template <typename T>
 void upload(Session& s) {
-    Packed<T> k = pack<T>(s.prep, s.cfg.uniform_prefix, s.cfg.rectangles, s.cfg.wavefront);
+    Packed<T> k = pack<T>(s.prep, s.cfg.uniform_prefix, s.cfg.rectangles, s.cfg.wavefront && s.cfg.nodes);
     size_t bytes = k.values.size() * sizeof(T) + k.guides.size() * sizeof(int);
     check(cudaMalloc(&s.scene, std::max<size_t>(bytes, 16)), "cudaMalloc(scene)");
     // Stream-ordered copies, complete before the host image goes out of scope.

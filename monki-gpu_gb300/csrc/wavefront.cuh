@@ -589,12 +589,12 @@ __device__ __forceinline__ int uniform_jump(const SceneView<T>& s, int& k, T& z,
 // One slot's walk to its next event: continues a split copy or claims a photon into an
 // empty slot (when claims are open), walks it, selects the interaction and stores the
 // state. Returns the event's queue (surface, gas, particle) or -1 when the slot holds no
-// event (empty or finished); with LISTS also kListPaused for a walk paused by the step budget
-// and kListVacant for an empty slot that can still be filled, which the caller lists. `given`
-// holds the slot's records when the caller has them in registers (a scattering just
-// made them); they are then not read back from memory. `claim` is the photon an empty slot takes
-// when the caller has reserved one for it, else kNone.
-template <typename T, bool PATHS, bool LISTS>
+// event (empty or finished), kListPaused for a walk paused by the step budget and kListVacant
+// for an empty slot that can still be filled; the caller lists the slot. `given` holds the
+// slot's records when the caller has them in registers (a scattering just made them); they are
+// then not read back from memory. `claim` is the photon an empty slot takes when the caller has
+// reserved one for it, else kNone.
+template <typename T, bool PATHS>
 __device__ __forceinline__ int transit_slot(uint32_t slot, const SceneView<T>& s, const T* band, const Controls& ctl,
                                             const Divisors& dv, const Pool<T>& P, uint32_t walk, bool may_claim,
                                             uint32_t* __restrict__ failure, uint64_t& scatters,
@@ -750,7 +750,7 @@ __device__ __forceinline__ int transit_slot(uint32_t slot, const SceneView<T>& s
         }
         if (PATHS && acc_k >= 0) path.add(acc_k, acc);
         if (outcome == 4) {  // budget spent: the walk resumes next iteration
-            if (LISTS) event = kListPaused;
+            event = kListPaused;
             break;
         }
         // A finished history leaves its slot empty until the next launch, where it is
@@ -792,7 +792,7 @@ __device__ __forceinline__ int transit_slot(uint32_t slot, const SceneView<T>& s
         if (meta.x != kNone || fresh) P.meta(slot) = make_uint4(kNone, 0u, 0u, 0u);
         // An empty slot waits for the next launch: copies still waiting keep it live; while
         // photons remain to claim it is refilled there.
-        return LISTS && ((P.waiting && P.waiting[slot] > 0u) || may_claim) ? kListVacant : -1;
+        return (P.waiting && P.waiting[slot] > 0u) || may_claim ? kListVacant : -1;
     }
     // The whole block, direction included (a scattering or a claim changed it; storing it
     // always also keeps every sector of the block fully written).
@@ -1432,9 +1432,10 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
     // room). 80-byte stride in FP32: the 16-byte accesses of a quarter warp fall in distinct
     // banks; 128 in FP64 for the 32-byte alignment of its records.
     constexpr int kHandStride = sizeof(T) == 4 ? 80 : 128;
-    __shared__ __align__(32) unsigned char hand[SCATTER && SMEM_HANDOFF ? 256 * kHandStride : 16];
+    constexpr bool kHandoff = SCATTER && SMEM_HANDOFF;
+    __shared__ __align__(32) unsigned char hand[kHandoff ? 256 * kHandStride : 16];
     SlotState<T> local_state;
-    SlotState<T>& state = SMEM_HANDOFF ? *reinterpret_cast<SlotState<T>*>(hand + threadIdx.x * kHandStride) : local_state;
+    SlotState<T>& state = kHandoff ? *reinterpret_cast<SlotState<T>*>(hand + threadIdx.x * kHandStride) : local_state;
     // One entry per thread: the lists hold at most one per slot, and the launch covers the pool or
     // (multi-scene sessions, every photon claimed) the entries read back since, whose number only
     // falls; a larger list was reported above. The loop stays all the same: outside of one the
@@ -1453,9 +1454,9 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
         } else {
             // The new records go to the walk through the handoff (it may also leave the slot vacant).
             if (SCATTER && scattered) scatter_event<T, NMAT, BACKWARD>(slot, surface, s, ctl, dv, P, g, failure, &state);
-            list = transit_slot<T, PATHS, true>(slot, s, band, ctl, dv, P, walk, may_claim, failure, scatters, visits,
-                                                SCATTER && scattered ? &state : nullptr,
-                                                e < walks || P.waiting ? kNone : first_claim + e);
+            list = transit_slot<T, PATHS>(slot, s, band, ctl, dv, P, walk, may_claim, failure, scatters, visits,
+                                          SCATTER && scattered ? &state : nullptr,
+                                          e < walks || P.waiting ? kNone : first_claim + e);
         }
     }
     // The block lists its slots with one reservation per list. Each counter is one address for
@@ -1629,8 +1630,7 @@ __device__ __forceinline__ void tail_phase(const SceneView<T>& s, const T* band,
             if (kind == kTailWalk ||
                 scatter_event<T, NMAT, BACKWARD>(slot, kind == kQueueSurface, s, ctl, dv, P, g, failure) ||
                 (P.waiting && P.waiting[slot] > 0u)) {
-                queue = transit_slot<T, PATHS, true>(slot, s, band, ctl, dv, P, kTailSteps, false, failure,
-                                                     scatters, visits);
+                queue = transit_slot<T, PATHS>(slot, s, band, ctl, dv, P, kTailSteps, false, failure, scatters, visits);
                 if (queue == kListVacant) queue = kTailWalk;  // its split copies next
             }
             if (queue >= 0) lists[cur ^ 1u][queue][warp_reserve(to, queue)] = slot;
