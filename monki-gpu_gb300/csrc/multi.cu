@@ -132,6 +132,7 @@ struct Scene {
     SceneView<float> view32{};
     SceneView<double> view64{};
     void* banks = nullptr;       // round_capacity x shards x W.count (T)
+    size_t bank_bytes = 0;
     double* out = nullptr;       // round_capacity x tally count (FP64, RawTallies order)
     double* info = nullptr;      // flush info: zunit, 1 / |mu0|, 1 / mu, mu0 / mu
     WaveTally W{};
@@ -168,6 +169,7 @@ struct Multi {
     uint32_t* tail_next = nullptr;             // one counter per scene for its tail launch
     std::vector<cudaStream_t> tail_streams;    // the scenes' tails run side by side
     size_t tail_used = 0;                      // taken in turn
+    bool unflushed = false;                    // a run failed between its transport and its flush
     cudaEvent_t t0 = nullptr, t1 = nullptr, t2 = nullptr;
     uint64_t totals[6] = {0, 0, 0, 0, 0, 0};
     float last_kernel_ms = 0.f, last_run_ms = 0.f;
@@ -574,9 +576,9 @@ void* monki_cuda_multi_create(uint32_t device, uint32_t scenes, const double* co
         for (Scene& sc : m->scenes) {
             const Prepared& p = sc.prep;
             if (cfg.fp64) upload_scene<double>(*m, sc, stream); else upload_scene<float>(*m, sc, stream);
-            const size_t bank = size_t(round_capacity) * sc.W.shards * sc.W.count * elem;
-            check(cudaMalloc(&sc.banks, bank), "cudaMalloc(banks)");
-            check(cudaMemsetAsync(sc.banks, 0, bank, stream), "cudaMemset(banks)");
+            sc.bank_bytes = size_t(round_capacity) * sc.W.shards * sc.W.count * elem;
+            check(cudaMalloc(&sc.banks, sc.bank_bytes), "cudaMalloc(banks)");
+            check(cudaMemsetAsync(sc.banks, 0, sc.bank_bytes, stream), "cudaMemset(banks)");
             check(cudaMalloc(&sc.out, size_t(round_capacity) * sc.tally_count * sizeof(double)), "cudaMalloc(out)");
             std::vector<double> info(size_t(p.nz) + 1 + 2 * size_t(p.angles));
             for (int z = 0; z < p.nz; ++z) info[size_t(z)] = p.zunit[size_t(z)];
@@ -634,6 +636,12 @@ int monki_cuda_multi_run(void* handle, const uint32_t* controls, double* const* 
         check(cudaMemsetAsync(m->failure, 0, sizeof(uint32_t), first), "memset(failure)");
         const size_t counter_bytes = m->scenes.size() * kSceneCounters * sizeof(unsigned long long);
         check(cudaMemsetAsync(m->counters, 0, counter_bytes, first), "memset(counters)");
+        if (m->unflushed) {
+            // The failed run's tallies are still in the banks (its last error was reported).
+            cudaGetLastError();
+            for (Scene& sc : m->scenes) check(cudaMemsetAsync(sc.banks, 0, sc.bank_bytes, first), "memset(banks)");
+        }
+        m->unflushed = true;
         check(cudaEventRecord(m->t0, first), "event");
         // Every group's stream starts after the clears above.
         for (Group& g : m->groups)
@@ -642,6 +650,7 @@ int monki_cuda_multi_run(void* handle, const uint32_t* controls, double* const* 
         for (Group& g : m->groups) check(cudaStreamSynchronize(g.stream), "multi-scene wavefront");
         check(cudaEventRecord(m->t1, first), "event");
         if (m->cfg.fp64) flush<double>(*m, ctl, first); else flush<float>(*m, ctl, first);
+        m->unflushed = false;
         check(cudaEventRecord(m->t2, first), "event");
         uint32_t flag = 0;
         std::vector<unsigned long long> cnt(m->scenes.size() * kSceneCounters, 0ull);

@@ -40,6 +40,8 @@ struct Session {
     cudaEvent_t t0 = nullptr, t1 = nullptr, t2 = nullptr;
     void* scene = nullptr;        // T values then int guides
     void* banks = nullptr;        // round_capacity x shards x tally count, TA
+    size_t bank_bytes = 0;
+    bool unflushed = false;       // a run failed between its transport and its flush
     double* out = nullptr;        // round_capacity x tally count
     double* mu0mu = nullptr;
     uint32_t* failure = nullptr;
@@ -433,6 +435,12 @@ void execute(Session& s, const Controls& c) {
     check(cudaSetDevice(s.device), "cudaSetDevice");
     check(cudaMemsetAsync(s.failure, 0, sizeof(uint32_t), s.stream), "memset(failure)");
     check(cudaMemsetAsync(s.counters, 0, 4 * sizeof(unsigned long long), s.stream), "memset(counters)");
+    if (s.unflushed) {
+        // The failed run's tallies are still in the banks (its last error was reported).
+        cudaGetLastError();
+        check(cudaMemsetAsync(s.banks, 0, s.bank_bytes, s.stream), "memset(banks)");
+    }
+    s.unflushed = true;
     const int needed = int(std::min<uint64_t>((uint64_t(c.count) + s.cfg.block - 1) / s.cfg.block, uint64_t(s.grid)));
     check(cudaEventRecord(s.t0, s.stream), "event");
     if (c.count) {
@@ -469,6 +477,7 @@ void execute(Session& s, const Controls& c) {
                 p.nx, p.ny, p.nz, p.angles, s.mu0mu, c.rounds, s.out);
         check(cudaGetLastError(), "flush launch");
     }
+    s.unflushed = false;
     check(cudaEventRecord(s.t2, s.stream), "event");
     s.totals[5] += 1;  // the flush
 }
@@ -603,9 +612,9 @@ void* monki_cuda_create(uint32_t device, const double* tables, size_t table_coun
         W.shards = cfg.shards;
         const size_t elem = cfg.fp64 ? sizeof(double) : sizeof(float);
         const size_t per_round = cfg.wavefront ? W.count : L.count;
-        const size_t bank_bytes = size_t(round_capacity) * L.shards * per_round * elem;
-        check(cudaMalloc(&s->banks, bank_bytes), "cudaMalloc(banks)");
-        check(cudaMemsetAsync(s->banks, 0, bank_bytes, s->stream), "cudaMemset(banks)");
+        s->bank_bytes = size_t(round_capacity) * L.shards * per_round * elem;
+        check(cudaMalloc(&s->banks, s->bank_bytes), "cudaMalloc(banks)");
+        check(cudaMemsetAsync(s->banks, 0, s->bank_bytes, s->stream), "cudaMemset(banks)");
         check(cudaMalloc(&s->out, size_t(round_capacity) * L.count * sizeof(double)), "cudaMalloc(out)");
         std::vector<double> mu(size_t(p.angles));
         // mu0/mu on forward Stokes tallies only (mc.f90:1456-1474).

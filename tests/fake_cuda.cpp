@@ -123,6 +123,9 @@ cudaError_t cudaMemsetAsync(void* p, int value, size_t n, cudaStream_t s) {
     std::memset(p, value, n);
     return emit("memset", "", s, p, n);
 }
+cudaError_t cudaMemcpy(void* dst, const void* src, size_t n, cudaMemcpyKind) { return copy("copy", dst, src, n, nullptr); }
+cudaError_t cudaMemset(void* p, int value, size_t n) { return cudaMemsetAsync(p, value, n, nullptr); }
+cudaError_t cudaGetSymbolAddress(void** p, const void* symbol) { *p = const_cast<void*>(symbol); return cudaSuccess; }
 cudaError_t cudaMemset2DAsync(void* p, size_t, int, size_t width, size_t height, cudaStream_t s) {
     return emit("memset", "", s, p, width * height);
 }

@@ -169,3 +169,18 @@ def test_a_tail_launch_lowers_no_other_sessions_shared_memory_limit(library):
     assert any(e.value > 0 for e in tails)  # a staged band
     assert {e.value for e in session.runtime.events if e.call == "attribute"} <= {48 * 1024}
     session.close()
+
+
+def test_a_run_after_a_failed_one_starts_from_empty_tallies(library):
+    session = Session(library, "pool=262144,check_every=2", live=((240000, 100), (330000, 200)))
+    banks = {(e.pointer, e.value) for e in session.runtime.events if e.call == "memset"}
+    assert len(banks) == 2
+    session.fail = lambda event: LAUNCH_FAILED if "wf_tail" in event.kernel else 0
+    assert session.run() == 1
+    session.fail = lambda event: 0
+    session.batches = [0, 0]
+    assert session.run() == 0, session.error.value
+    events = session.of_run()
+    started = next(n for n, e in enumerate(events) if "wf_" in e.kernel)
+    assert banks <= {(e.pointer, e.value) for e in events[:started] if e.call == "memset"}
+    session.close()
