@@ -70,7 +70,6 @@ E2E_ROUNDS = 32  # rounds of the end-to-end run at the workload's own round size
 STATE_BYTES = 64  # one event's photon state records read by the peel kernel
 CELL_BYTES = 16  # one cell record (beta + cumulative species fractions)
 TALLY_BYTES = 32  # one 128-bit tally atomic: 16 B read + 16 B written in L2
-SLOT_SCAN_BYTES = 16  # transit reads every slot's bookkeeping record
 TRANSIT_EVENT_BYTES = 109  # per event: state read (52 B) and written (52 B), queue entry and kind (5 B)
 SCATTER_EVENT_BYTES = 116  # per event: queue entry (4 B), state read (64 B) and written (48 B)
 # Fused step (scenes without layer paths): per event its list entry (4 B), its state read once
@@ -92,8 +91,8 @@ def peaks():
 
 def recorded_traffic(workload, kernel, per_launch=None):
     """Per-launch DRAM bytes (read + write) of one wavefront kernel from the committed ncu
-    summary of the workload, or None. The captures ran a smaller pool than the bench's
-    launches; when the summary gives the algorithmic bytes of the captured launch, its
+    summary of the workload, or None. The captures ran fewer photons per column than the
+    bench's launches; when the summary gives the algorithmic bytes of the captured launch, its
     traffic is scaled to this launch by the algorithmic bytes (the units processed): the
     traffic grows with the events a launch handles."""
 
@@ -605,8 +604,8 @@ def main():
     # launch duration; the line reports the kernel with the largest share of device time.
     #   step     (scenes without layer paths) each event's list entry, its state read once
     #            and written once, its new queue entry, 16 B per free-path cell visit
-    #   transit  every slot's bookkeeping record, each event's state read and written and
-    #            its queue entry, 16 B per free-path cell visit
+    #   transit  each event's state read and written and its queue entry, 16 B per
+    #            free-path cell visit
     #   peel     each event's state, 16 B per detector-ray cell visit, 32 B per tally atomic
     #   scatter  each event's queue entry and state read and written
     peak, peak_kind = peaks()
@@ -614,10 +613,9 @@ def main():
     fused = not scene.save_path  # the session's default: fused step unless the scene has layer paths
     names = ("step", "peel") if fused else ("transit", "peel", "scatter")
     stage_share = {name: stage_ms[q] / stage_total for q, name in enumerate(names)}
-    pool = 1 << 22  # the session's default pool (every slot scanned by a transit launch)
     algorithmic = {
         "step": STEP_EVENT_BYTES * p_scatters + CELL_BYTES * p_visits_fp,
-        "transit": SLOT_SCAN_BYTES * pool * int(stage_launches[0]) + TRANSIT_EVENT_BYTES * p_scatters + CELL_BYTES * p_visits_fp,
+        "transit": TRANSIT_EVENT_BYTES * p_scatters + CELL_BYTES * p_visits_fp,
         "peel": STATE_BYTES * p_scatters + CELL_BYTES * p_visits_det + TALLY_BYTES * p_updates,
         "scatter": SCATTER_EVENT_BYTES * p_scatters,
     }

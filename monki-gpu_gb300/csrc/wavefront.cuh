@@ -2,7 +2,7 @@
 // stage of a history runs as its own kernel over event queues, so a warp always executes
 // one kind of work.
 //
-//   transit  walks every pooled photon along its free path (ADVANCE, mc.f90:1531-1580)
+//   transit  walks every listed photon along its free path (ADVANCE, mc.f90:1531-1580)
 //            to its next interaction, draws the species and applies the single-scattering
 //            albedo (mc.f90:1028-1074) or the surface albedo (mc.f90:681-728), and appends
 //            the photon to the surface / gas / particle queue. Slots whose photon escaped or
@@ -584,7 +584,7 @@ __device__ __forceinline__ int uniform_jump(const SceneView<T>& s, int& k, T& z,
 }
 
 // ----------------------------------------------------------------------------------
-// transit: free path to the next interaction for every pooled photon.
+// transit: free path to the next interaction for every listed photon.
 // ----------------------------------------------------------------------------------
 // One slot's walk to its next event: continues a split copy or claims a photon into an
 // empty slot (when claims are open), walks it, selects the interaction and stores the
@@ -1461,9 +1461,9 @@ __device__ __forceinline__ void step_phase(const SceneView<T>& s, const T* band,
     }
     // The block lists its slots with one reservation per list. Each counter is one address for
     // the whole launch, where atomics are served one after the other: a reservation per warp
-    // and list took 0.5 ms of turns per launch of the full pool, about the kernel's whole time.
-    // Clear sky, 32 rounds of 2,000 photons per column 45.3 -> 37.6 ms; box cloud, a round of
-    // 50,000 126.2 -> 108.5 ms.
+    // and list took a quarter of the kernel (clear sky, a launch of the full pool 510 -> 385 us).
+    // Whole calls: clear sky, 32 rounds of 2,000 photons per column 45.3 -> 37.6 ms; box cloud, a
+    // round of 50,000 126.2 -> 108.5 ms.
     const uint32_t offset = list >= 0 ? warp_reserve(listed, list) : 0u;
     __syncthreads();
     if (threadIdx.x < kLists && listed[threadIdx.x])
@@ -1558,8 +1558,11 @@ constexpr int kTailBlock = 256;
 constexpr int kTailWarps = kTailBlock / 32;
 constexpr int kTailWalk = kListPaused;  // list of the slots that walk on without a scattering
 // Walk steps per photon and iteration, like the step's budget: a block waits for its longest
-// walk, and walks that go on share warps of their own in the next iteration (pilot run, two
-// rounds of 300 photons per column: 13.65 ms unlimited, 13.4 at 6 steps, 13.2 at 3).
+// walk, and walks that go on share warps of their own in the next iteration. Three is the
+// fastest or level for every kind of scene; whole calls in ms at 1 / 3 / 6 / unlimited: pilot
+// run, two rounds of 300 photons per column 13.05 / 12.87 / 13.18 / 13.17; box cloud, one round of
+// 1,000 8.52 / 8.47 / 8.68 / 8.69; backward, two rounds of 2,000 8.49 / 8.37 / 8.42 / 8.42;
+// layered cloud and clear sky level.
 constexpr uint32_t kTailSteps = 3;
 
 template <typename T, int NMAT, bool PATHS, bool BACKWARD>
